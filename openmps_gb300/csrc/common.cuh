@@ -155,8 +155,9 @@ struct DeviceState {
 //      each way bring 0 <= R < mb (0 <= R <= 2S for the root), and the quotient or root
 //      rounds up when 2R > mb (R > S); ties cannot occur for a quotient or a root of
 //      53-bit significands.
-// Operands that are zero, subnormal, infinite or NaN, and results outside the normal
-// range, take __ddiv_rn / __dsqrt_rn, so every input gives the IEEE result.
+// A zero divided by a normal number is that signed zero.  Other operands that are zero,
+// subnormal, infinite or NaN, and results outside the normal range, take __ddiv_rn /
+// __dsqrt_rn, so every input gives the IEEE result.
 namespace exact {
 
 constexpr unsigned long long kM52 = (1ull << 52) - 1ull, kH52 = 1ull << 52;
@@ -213,7 +214,13 @@ __device__ __forceinline__ double ddiv_rn(double a, double b) {
         e++;
     }
     const bool fast = ea != 0 && ea != 2047 && eb != 0 && eb != 2047 && e >= 1 && e <= 2046 && in_range;
-    if (!fast) return __ddiv_rn(a, b);
+    if (!fast) {
+        // a zero numerator is common in earnest (the pressure gradient divides p_i + p_j,
+        // zero at and near a free surface): the quotient by a normal number is a zero with
+        // the sign of the operands, without the FP64 routine
+        if ((ua << 1) == 0ull && eb != 0 && eb != 2047) return __longlong_as_double(static_cast<long long>((ua ^ ub) & (1ull << 63)));
+        return __ddiv_rn(a, b);
+    }
     return __longlong_as_double(static_cast<long long>(((ua ^ ub) & (1ull << 63)) |
                                                        (static_cast<unsigned long long>(e) << 52) |
                                                        (static_cast<unsigned long long>(Q) & kM52)));
