@@ -32,6 +32,7 @@ UNITS = {
     "stages.cu": ["-fmad=false"],
     "dim3.cu": ["-fmad=false"],
     "cg.cu": [],
+    "cgloop.cu": [],
     "mg.cu": [],
     "learned.cu": [],
     "batch.cu": [],

@@ -1,8 +1,10 @@
 // cg.cu - pressure Poisson solvers (Computer::SolvePressurePoissonEquation,
-// Computer.hpp:1359-1429) on the SELL-32 matrix, each run as one CUDA graph: an init
-// kernel, then a conditional WHILE node whose body is a few kernels; the last block of
-// each reduction decides the next step and sets the graph condition, so a solve of
-// thousands of iterations needs no host round trip.
+// Computer.hpp:1359-1429) on the SELL-32 matrix, each run as one CUDA graph: init kernels,
+// then the iterations: one launch for the plain solvers (cgloop.cu), a conditional WHILE node
+// whose body is a few kernels for the preconditioned ones; the last block of each reduction
+// decides the next step and sets the graph condition, so a solve of thousands of iterations
+// needs no host round trip.  With MPS_CG_LAUNCH_HOST every phase of every solver is launched
+// by the host.
 //
 // Work layout: vector kernels run one thread per row, SpMV kernels one warp per chunk of
 // 32 rows (one lane per row, as many warps as chunks, so the block scheduler balances
@@ -18,22 +20,20 @@
 // the group's, and the last group adds the group sums (atomic tickets, no waiting).  Every
 // addition has a fixed order, so results are deterministic run to run.
 //
-// MPS_SOLVER_CG64: the reference CG in FP64 (3 kernels per iteration).
+// MPS_SOLVER_CG64: the reference CG in FP64 (3 kernels per iteration from the host).
 // MPS_SOLVER_MIXED: CG whose iterations run in FP32 (FP32 matrix, FP32 SpMV and axpy with
 // FP32 accumulation, dot products accumulated in FP64) with reliable updates (Sleijpen &
 // van der Vorst 1996): when the recursive residual has dropped by `delta` since the last
 // update, the FP32 correction is folded into the FP64 solution and the true residual
-// b - A x is recomputed with the FP64 matrix, which also decides convergence.  The
-// direction update p = r + beta p is folded into the next SpMV (each lane forms
-// beta p_j + r_j while gathering), so an iteration is two kernels; the reliable update
-// runs under a conditional IF node only when due.
+// b - A x is recomputed with the FP64 matrix, which also decides convergence.
 // MPS_SOLVER_MIXED_MG / LEARNED: the same FP32 iteration preconditioned by the cell
 // multigrid (mg.cu), three dot products per reduction; if it stalls or runs out of
 // iterations the plain FP64 CG continues from the solution it reached, inside the same
-// graph (a second WHILE node that runs zero times after a converged solve).
+// graph (its loop launch returns at once after a converged solve).
 #include <cmath>
 #include <vector>
 
+#include "gridloop.cuh"
 #include "learned.cuh"
 
 namespace mpsgb {
@@ -201,22 +201,30 @@ __device__ __forceinline__ bool aborted_before_solve(const CgOperands& o,
     return false;
 }
 
+// The width of chunk c for the single-launch loops, or 0 when they leave it out: every row
+// is an identity row (its diagonal alone) with a zero residual, so its x stays.  Warp per
+// chunk, lane = row i of length L at `at`, residual ri.
+__device__ __forceinline__ void store_loop_width(const CgOperands& o, int c, int i, int L, int64_t at, double ri) {
+    const bool idle = L == 0 || (L == 1 && o.col[at] == i && ri == 0.0);
+    const bool out = __all_sync(kFull, idle);
+    if ((threadIdx.x & 31) == 0 && o.loop_w) o.loop_w[c] = out ? 0 : o.chunk[c] / kSellRows;
+}
+
 // ------------------------------------------------------------- CG64 kernels
 // Ap = A x; r = b - Ap; p = r; rr = r.r (Computer.hpp:1382-1385).  With `gate` (the
 // fallback after a preconditioned solve) nothing runs unless that solve failed.
-__global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, cudaGraphConditionalHandle h,
-                                                   int use_cond, const CgScalars* gate) {
+__global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, const CgScalars* gate) {
     __shared__ BlockTicket tk;
     if (gate && (gate->converged || gate->aborted)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             o.S->converged = gate->converged;
             o.S->aborted = gate->aborted;
             o.S->iter = 0;
-            if (use_cond) cudaGraphSetConditional(h, 0u);
         }
         return;
     }
-    if (aborted_before_solve(o, h, use_cond)) return;
+    if (aborted_before_solve(o, 0, 0)) return;
+    clear_slots(o.slots);
     ticket_init(tk);
     const ChunkLoop cl;
     const double* x = o.x;
@@ -224,51 +232,25 @@ __global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, cudaGraphCondi
     for (int c = cl.warp; c < o.nchunks; c += cl.nwarps) {
         const int i = kSellRows * c + cl.lane;
         const int L = o.len[i];
-        const double ax = row64(o, sell_index(o.off[c], cl.lane, 0), L, [&](int j) { return x[j]; });
+        const int64_t at = sell_index(o.off[c], cl.lane, 0);
+        const double ax = row64(o, at, L, [&](int j) { return x[j]; });
+        double ri = 0.0;
         if (i < o.n) {
             const double bi = o.b[i];
-            const double ri = bi - ax;
+            ri = bi - ax;
             o.r[i] = ri;
             o.p[i] = ri;
             vrr += ri * ri;
             vbb += bi * bi;
         }
+        store_loop_width(o, c, i, L, at, ri);
     }
     double tot[3];
-    if (grid_sum(vrr, vbb, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) init_scalars(o.S, tot[0], tot[1], h, use_cond);
-}
-
-// Ap = A p; alpha = rr / (p.Ap)
-__global__ void __launch_bounds__(kBlock) k_cg_spmv_dot(CgOperands o) {
-    __shared__ BlockTicket tk;
-    if (cg_done(o.S)) return;
-    ticket_init(tk);
-    const ChunkLoop cl;
-    const double* p = o.p;
-    double v = 0.0;
-    for (int c = cl.warp; c < o.nchunks; c += cl.nwarps) {
-        const int i = kSellRows * c + cl.lane;
-        const int L = o.len[i];
-        const double s = row64(o, sell_index(o.off[c], cl.lane, 0), L, [&](int j) { return p[j]; });
-        if (i < o.n) {
-            o.Ap[i] = s;
-            v += p[i] * s;
-        }
-    }
-    double tot[3];
-    if (grid_sum(v, 0.0, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) {
-        const double pap = tot[0];
-        {
-            o.S->counter = 0;
-            o.S->pAp = pap;
-            o.S->alpha = o.S->rr / pap;
-        }
-    }
+    if (grid_sum(vrr, vbb, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) init_scalars(o.S, tot[0], tot[1], 0, 0);
 }
 
 // x += alpha p; r -= alpha Ap; rrNew = r.r; convergence; beta (Computer.hpp:1402-1420)
-__global__ void __launch_bounds__(kBlock) k_cg_update(CgOperands o, cudaGraphConditionalHandle h,
-                                                     int use_cond) {
+__global__ void __launch_bounds__(kBlock) k_cg_update(CgOperands o) {
     __shared__ BlockTicket tk;
     if (cg_done(o.S)) return;
     ticket_init(tk);
@@ -294,7 +276,6 @@ __global__ void __launch_bounds__(kBlock) k_cg_update(CgOperands o, cudaGraphCon
                 S->rr = rr_new;
             }
             S->iter += 1;
-            if (use_cond) cudaGraphSetConditional(h, (!conv && S->iter < S->max_iter) ? 1u : 0u);
         }
     }
 }
@@ -345,10 +326,12 @@ __global__ void __launch_bounds__(kBlock) k_true_residual(CgOperands o, int afte
 // followed by the SpMV w = A r that also forms gamma and delta and the next step sizes.
 
 // init: r_0 = b - A x (FP64); r32 = r_0; d = 0; p = 0; s = 0; rr, bb
+// (plain: MIXED, whose loop leaves some rows out: both solution buffers hold their x)
 __global__ void __launch_bounds__(kBlock) k_mx_init(CgOperands o, cudaGraphConditionalHandle h,
-                                                   int use_cond) {
+                                                   int use_cond, int plain) {
     __shared__ BlockTicket tk;
     if (aborted_before_solve(o, h, use_cond)) return;
+    clear_slots(o.slots);
     ticket_init(tk);
     const ChunkLoop cl;
     const double* x = o.x;
@@ -356,10 +339,13 @@ __global__ void __launch_bounds__(kBlock) k_mx_init(CgOperands o, cudaGraphCondi
     for (int c = cl.warp; c < o.nchunks; c += cl.nwarps) {
         const int i = kSellRows * c + cl.lane;
         const int L = o.len[i];
-        const double ax = row64(o, sell_index(o.off[c], cl.lane, 0), L, [&](int j) { return x[j]; });
+        const int64_t at = sell_index(o.off[c], cl.lane, 0);
+        const double ax = row64(o, at, L, [&](int j) { return x[j]; });
+        double ri = 0.0;
         if (i < o.n) {
             const double bi = o.b[i];
-            const double ri = bi - ax;
+            ri = bi - ax;
+            if (plain) o.x2[i] = x[i];
             o.r32[i] = __double2float_rn(ri);
             o.s32[i] = 0.0f;
             o.p32[i] = 0.0f;
@@ -368,6 +354,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_init(CgOperands o, cudaGraphCondi
             vrr += ri * ri;
             vbb += bi * bi;
         }
+        if (plain) store_loop_width(o, c, i, L, at, ri);
     }
     double tot[3];
     if (grid_sum(vrr, vbb, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) init_scalars(o.S, tot[0], tot[1], h, use_cond);
@@ -392,14 +379,7 @@ __global__ void __launch_bounds__(kBlock) k_mx_axpy(CgOperands o) {
 // w = A r (FP32); gamma = r.r and delta = w.r in FP64; the next Chronopoulos-Gear step
 // sizes; decides a reliable update.  mode 0: after init (beta = 0); mode 1: an
 // iteration; mode 2: after a reliable update (also clears d, folded into x).
-// Iterations the plain mixed solver may run without a reliable update (a tenfold drop of
-// its recursive residual norm takes a few hundred iterations on the PPEs of the
-// workloads when the FP32 recursion makes progress).
-constexpr int kMixedStallIter = 2000;
-
-__global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode,
-                                                   cudaGraphConditionalHandle h,
-                                                   cudaGraphConditionalHandle h_true, int use_cond) {
+__global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode) {
     __shared__ BlockTicket tk;
     CgScalars* S = o.S;
     if (mode == 2) {
@@ -436,7 +416,6 @@ __global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode,
             if (mode == 1) {
                 reliable = (gam < S->delta2 * S->rr_upd) || (gam < S->thr);
                 S->do_update = reliable;
-                if (use_cond && h_true) cudaGraphSetConditional(h_true, reliable ? 1u : 0u);
             }
             if (!reliable) {
                 if (mode == 0) {
@@ -451,7 +430,6 @@ __global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode,
                     // iterations: the FP32 iteration has stalled (the FP64 CG takes over)
                     const int stuck = S->iter - S->iter_upd > kMixedStallIter;
                     if (stuck) S->stalled = 1;
-                    if (use_cond) cudaGraphSetConditional(h, (!stuck && S->iter < S->max_iter) ? 1u : 0u);
                 }
                 S->rr = gam;
                 S->pAp = del;
@@ -463,14 +441,11 @@ __global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode,
                 S->prev_true_rr = S->true_rr;
                 S->stalled = stalled;
                 S->do_update = 0;
-                if (use_cond && stalled) cudaGraphSetConditional(h, 0u);
             }
         }
     }
 }
 
-// Reliable update, part 1: x' = x + d and r = b - A x' in FP64 (FP64 matrix), written
-// over the r the iteration produced; convergence on this true residual.
 // The scalars after a reliable update's true residual r.r: the new reference for the
 // next update, and convergence (which ends the loop).
 __device__ __forceinline__ void true_residual_done(CgScalars* S, double rr, cudaGraphConditionalHandle h,
@@ -485,37 +460,6 @@ __device__ __forceinline__ void true_residual_done(CgScalars* S, double rr, cuda
     if (conv) {
         S->iter += 1;
         if (use_cond) cudaGraphSetConditional(h, 0u);
-    }
-}
-
-__global__ void __launch_bounds__(kBlock) k_mx_true(CgOperands o, cudaGraphConditionalHandle h,
-                                                   int use_cond) {
-    __shared__ BlockTicket tk;
-    if (o.S->converged || o.S->aborted || o.S->stalled || !o.S->do_update) return;
-    ticket_init(tk);
-    const ChunkLoop cl;
-    const bool odd = (o.S->updates & 1) != 0;
-    const double* __restrict__ xc = odd ? o.x2 : o.x;
-    double* __restrict__ xn = odd ? o.x : o.x2;
-    const float* __restrict__ d = o.d32;
-    float* __restrict__ rslot = o.r32;
-    double v = 0.0;
-    for (int c = cl.warp; c < o.nchunks; c += cl.nwarps) {
-        const int i = kSellRows * c + cl.lane;
-        const int L = o.len[i];
-        const double ax = row64(o, sell_index(o.off[c], cl.lane, 0), L,
-                                [&](int j) { return xc[j] + static_cast<double>(d[j]); });
-        if (i < o.n) {
-            const double ri = o.b[i] - ax;
-            xn[i] = xc[i] + static_cast<double>(d[i]);
-            rslot[i] = __double2float_rn(ri);
-            v += ri * ri;
-        }
-    }
-    double tot[3];
-    if (grid_sum(v, 0.0, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) {
-        o.S->counter = 0;
-        true_residual_done(o.S, tot[0], h, use_cond);
     }
 }
 
@@ -762,11 +706,11 @@ struct StageRing {
 };
 
 // What a staged FP64 SpMV computes: the CG's A p (with p.Ap and the step size alpha =
-// rr / p.Ap, as k_cg_spmv_dot), or the mixed solves' true residual r = b - A x' after a
+// rr / p.Ap), or the mixed solves' true residual r = b - A x' after a
 // reliable update folded the FP32 correction into x' (with r.r and the update's decisions).
 enum StagedKind { kStagedCgAp = 0, kStagedTrueResidual = 1 };
 
-// k_cg_spmv_dot with the staged stream.  A lane sums its row from the stages in
+// A lane sums its row from the stages in
 // ascending column order with one accumulator (the order of row64), so the row sums are
 // those of the per-chunk kernel.
 template <int SLICE, int STAGES, int MINB, int KIND>
@@ -884,36 +828,27 @@ constexpr size_t kStgSmem64 = static_cast<size_t>(kStgWarps) * kStgStages64 * (k
 // cg_prepare_device before any launch or capture
 int g_stg_per_sm64 = 1;
 
-// the FP64 CG's SpMV (Ap = A p, p.Ap, alpha): staged when the handle gives an SM count
+int staged_grid(const CgOperands& o) {
+    const int cap = o.grid_staged * g_stg_per_sm64;
+    const int need = (o.nchunks + kStgWarps - 1) / kStgWarps;
+    return need < cap ? (need > 0 ? need : 1) : cap;
+}
+
+// the FP64 CG's SpMV (Ap = A p, p.Ap, alpha)
 void launch_cg_spmv(const CgOperands& o, cudaStream_t s) {
-    if (o.grid_staged > 0) {
-        const int cap = o.grid_staged * g_stg_per_sm64;
-        const int need = (o.nchunks + kStgWarps - 1) / kStgWarps;
-        const int g = need < cap ? (need > 0 ? need : 1) : cap;
-        k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedCgAp>
-            <<<g, kStgThreads, kStgSmem64, s>>>(o, 0, 0);
-        return;
-    }
-    k_cg_spmv_dot<<<o.grid_spmv, kBlock, 0, s>>>(o);
+    k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedCgAp>
+        <<<staged_grid(o), kStgThreads, kStgSmem64, s>>>(o, 0, 0);
 }
 
 // A reliable update's true residual: the fold x' = x + d and the staged FP64 SpMV
-// r = b - A x' (about 50 us at 340k), or, without an SM count, one per-chunk kernel that
-// gathers x + d on the fly.
+// r = b - A x' (about 50 us at 340k).
 void launch_mx_true(const CgOperands& o, cudaGraphConditionalHandle h, int use_cond, cudaStream_t s) {
-    if (o.grid_staged > 0) {
-        const int cap = o.grid_staged * g_stg_per_sm64;
-        const int need = (o.nchunks + kStgWarps - 1) / kStgWarps;
-        const int g = need < cap ? (need > 0 ? need : 1) : cap;
-        k_mx_fold<<<o.grid_vec, kBlock, 0, s>>>(o);
-        k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedTrueResidual>
-            <<<g, kStgThreads, kStgSmem64, s>>>(o, h, use_cond);
-        return;
-    }
-    k_mx_true<<<o.grid_spmv, kBlock, 0, s>>>(o, h, use_cond);
+    k_mx_fold<<<o.grid_vec, kBlock, 0, s>>>(o);
+    k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedTrueResidual>
+        <<<staged_grid(o), kStgThreads, kStgSmem64, s>>>(o, h, use_cond);
 }
 
-int mx_true_launches(const CgOperands& o) { return o.grid_staged > 0 ? 2 : 1; }
+constexpr int kMxTrueLaunches = 2;
 
 // the preconditioned FP32 SpMV (w = A u, three dot products)
 void launch_pmx_spmv(const CgOperands& o, int mode, cudaGraphConditionalHandle h, cudaGraphConditionalHandle h_true,
@@ -1257,9 +1192,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_pcg_persistent(CgOperands o, MgHi
 
 bool is_pcg(int solver) { return solver == MPS_SOLVER_MIXED_MG || solver == MPS_SOLVER_LEARNED; }
 
-void cg64_body(const CgOperands& ops, cudaGraphConditionalHandle h, int use_cond, cudaStream_t s) {
+void cg64_body(const CgOperands& ops, cudaStream_t s) {
     launch_cg_spmv(ops, s);
-    k_cg_update<<<ops.grid_vec, kBlock, 0, s>>>(ops, h, use_cond);
+    k_cg_update<<<ops.grid_vec, kBlock, 0, s>>>(ops);
     k_cg_pupdate<<<ops.grid_vec, kBlock, 0, s>>>(ops);
 }
 
@@ -1270,7 +1205,7 @@ void reliable_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
         mg_apply(*mg, ops.S, 2, ops.r32, ops.u32, s);
         launch_pmx_spmv(ops, 2, h, 0, use_cond, s, false);
     } else {
-        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops, 2, h, 0, use_cond);
+        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops, 2);
     }
 }
 
@@ -1279,7 +1214,7 @@ void body_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
                   bool with_true, cudaStream_t s) {
     const int gv = ops.grid_vec, gs = ops.grid_spmv;
     if (solver == MPS_SOLVER_CG64) {
-        cg64_body(ops, h, use_cond, s);
+        cg64_body(ops, s);
         return;
     }
     if (is_pcg(solver)) {
@@ -1287,7 +1222,7 @@ void body_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
         launch_pmx_spmv(ops, 1, h, h_true, use_cond, s, true);
     } else {
         k_mx_axpy<<<gv, kBlock, 0, s>>>(ops);
-        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops, 1, h, h_true, use_cond);
+        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops, 1);
     }
     if (with_true) reliable_kernels(solver, ops, mg, h, use_cond, s);
 }
@@ -1298,7 +1233,7 @@ void body_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
 void learned_prep_head(const LearnedOps& L, const CgOperands& o, CgScalars* S, cudaStream_t s) {
     CgOperands p = o;
     p.S = S;
-    k_mx_init<<<o.grid_spmv, kBlock, 0, s>>>(p, 0, 0);  // r0 = b - A x0 in FP64, into r32
+    k_mx_init<<<o.grid_spmv, kBlock, 0, s>>>(p, 0, 0, 0);  // r0 = b - A x0 in FP64, into r32
     launch_learned_q(L, p, S, s);
 }
 
@@ -1325,7 +1260,7 @@ void init_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
                   const LearnedRun* lrn, const SetupFork* fk = nullptr) {
     const int gs = ops.grid_spmv;
     if (solver == MPS_SOLVER_CG64) {
-        k_cg_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, nullptr);
+        k_cg_init<<<gs, kBlock, 0, s>>>(ops, nullptr);
         return;
     }
     const bool pcg = is_pcg(solver);
@@ -1346,16 +1281,16 @@ void init_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
         learned_prep_head(*lrn->L, ops, lrn->S, s);
         if (forked) cudaStreamWaitEvent(s, fk->join, 0);
         learned_prep_tail(*lrn->L, ops, *mg, lrn->S, true, s);
-        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond);
+        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, pcg ? 0 : 1);
     } else {
-        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond);
+        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, pcg ? 0 : 1);
         if (forked) cudaStreamWaitEvent(s, fk->join, 0);
     }
     if (pcg) {
         mg_apply(*mg, ops.S, 0, ops.r32, ops.u32, s);
         launch_pmx_spmv(ops, 0, h, 0, use_cond, s, false);
     } else {
-        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops, 0, h, 0, use_cond);
+        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops, 0);
     }
 }
 
@@ -1375,7 +1310,7 @@ cudaError_t cg_prepare_device() {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, kStgThreads, kStgSmem64);
     if (e != cudaSuccess) return e;
     g_stg_per_sm64 = b > 0 ? b : 1;
-    return cudaSuccess;
+    return cg_loop_prepare_device();
 }
 
 int64_t cg_partials(int64_t n) {
@@ -1400,7 +1335,7 @@ void launch_spmv_only(int solver, const CgOperands& ops, cudaStream_t s) {
     else if (is_pcg(solver))
         launch_pmx_spmv(ops, 1, 0, 0, 0, s, false);
     else
-        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops, 1, 0, 0, 0);
+        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops, 1);
 }
 
 void learned_prep(const LearnedOps& L, const CgOperands& o, const MgHierarchy& mg, CgScalars* S,
@@ -1418,10 +1353,9 @@ int cg_kernels_per_iteration(int solver, const MgHierarchy* mg) {
     return is_pcg(solver) && mg ? 1 + mg_apply_launches(*mg) : 2;
 }
 
-int cg_kernels_per_update(int solver, const MgHierarchy* mg, const CgOperands& ops) {
+int cg_kernels_per_update(int solver, const MgHierarchy* mg) {
     if (solver == MPS_SOLVER_CG64) return 0;
-    const int t = mx_true_launches(ops);
-    return is_pcg(solver) && mg ? t + 1 + mg_apply_launches(*mg) : t + 1;
+    return is_pcg(solver) && mg ? kMxTrueLaunches + 1 + mg_apply_launches(*mg) : kMxTrueLaunches + 1;
 }
 
 CgGraph::~CgGraph() {
@@ -1443,14 +1377,58 @@ void CgGraph::reset() {
 
 cudaError_t CgGraph::build(int solver, const CgOperands& ops, cudaStream_t s, const MgHierarchy* mg,
                            const CgOperands* fb, const LearnedRun* lrn) {
-    if (is_pcg(solver) && (!mg || !fb)) return cudaErrorInvalidValue;
+    if (!is_pcg(solver)) return build_plain(solver, ops, s, fb);
+    if (!mg || !fb) return cudaErrorInvalidValue;
     if (solver == MPS_SOLVER_LEARNED && !lrn) return cudaErrorInvalidValue;
-    if (solver != MPS_SOLVER_CG64) {
-        // preferred: the reliable update under an IF node nested in the WHILE body
-        if (build_impl(solver, ops, s, true, mg, fb, lrn) == cudaSuccess) return cudaSuccess;
-        cudaGetLastError();
-    }
+    // preferred: the reliable update under an IF node nested in the WHILE body
+    if (build_impl(solver, ops, s, true, mg, fb, lrn) == cudaSuccess) return cudaSuccess;
+    cudaGetLastError();
     return build_impl(solver, ops, s, false, mg, fb, lrn);
+}
+
+namespace {
+// After a mixed-precision loop: the plain FP64 CG from the solution reached, which runs
+// only if that loop failed, then the statistics' true residual.
+cudaError_t fallback_kernels(const CgOperands& ops, const CgOperands& fb, int after_update, cudaStream_t s) {
+    k_cg_init<<<fb.grid_spmv, kBlock, 0, s>>>(fb, ops.S);
+    const cudaError_t e = launch_cg_loop(fb, s);
+    k_fb_merge<<<1, 32, 0, s>>>(ops.S, fb.S);
+    k_true_residual<<<ops.grid_spmv, kBlock, 0, s>>>(ops, after_update);
+    return e;
+}
+}  // namespace
+
+// CG64 and MIXED: init, the loop in one launch (cgloop.cu), [the FP64 CG after a failed
+// mixed loop], the true residual.
+cudaError_t CgGraph::build_plain(int solver, const CgOperands& ops, cudaStream_t s, const CgOperands* fb) {
+    reset();
+    ops_ = ops;
+    solver_ = solver;
+    cudaError_t e = cudaGraphCreate(&graph_, 0);
+    if (e != cudaSuccess) return e;
+    cudaGraph_t captured = nullptr;
+    e = cudaStreamBeginCaptureToGraph(s, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    init_kernels(solver, ops, nullptr, 0, 0, s, nullptr);
+    cudaError_t le;
+    if (solver == MPS_SOLVER_CG64) {
+        le = launch_cg_loop(ops, s);
+    } else {
+        le = launch_mx_loop(ops, s);
+        k_mx_finish<<<ops.grid_vec, kBlock, 0, s>>>(ops);
+    }
+    if (solver != MPS_SOLVER_CG64 && fb) {
+        const cudaError_t fe = fallback_kernels(ops, *fb, 1, s);
+        if (le == cudaSuccess) le = fe;
+    } else {
+        k_true_residual<<<ops.grid_spmv, kBlock, 0, s>>>(ops, solver != MPS_SOLVER_CG64 ? 1 : 0);
+    }
+    e = cudaStreamEndCapture(s, &captured);
+    if (le != cudaSuccess) return le;
+    if (e != cudaSuccess) return e;
+    e = cudaGraphInstantiate(&exec_, graph_, 0);
+    if (e != cudaSuccess) exec_ = nullptr;
+    return e;
 }
 
 namespace {
@@ -1505,19 +1483,12 @@ cudaError_t CgGraph::build_impl(int solver, const CgOperands& ops, cudaStream_t 
     solver_ = solver;
     nested_ = nested;
     kpi_ = cg_kernels_per_iteration(solver, mg);
-    kri_ = cg_kernels_per_update(solver, mg, ops);
-    const int gv = ops.grid_vec, gs = ops.grid_spmv;
+    kri_ = cg_kernels_per_update(solver, mg);
     cudaError_t e = cudaGraphCreate(&graph_, 0);
     if (e != cudaSuccess) return e;
-    cudaGraphConditionalHandle h, h_fb = 0;
+    cudaGraphConditionalHandle h;
     e = cudaGraphConditionalHandleCreate(&h, graph_, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return e;
-    // the mixed-precision solvers end with the plain FP64 CG when they stall
-    const bool with_fb = solver != MPS_SOLVER_CG64 && fb != nullptr;
-    if (with_fb) {
-        e = cudaGraphConditionalHandleCreate(&h_fb, graph_, 0, cudaGraphCondAssignDefault);
-        if (e != cudaSuccess) return e;
-    }
     cudaGraph_t captured = nullptr;
 
     // init chain (the multigrid's coarse setup on a side branch)
@@ -1579,36 +1550,11 @@ cudaError_t CgGraph::build_impl(int solver, const CgOperands& ops, cudaStream_t 
     e = cudaStreamBeginCaptureToGraph(s, graph_, &while_node, nullptr, 1,
                                       cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    if (solver != MPS_SOLVER_CG64) k_mx_finish<<<gv, kBlock, 0, s>>>(ops);
-    if (with_fb) {
-        k_cg_init<<<gs, kBlock, 0, s>>>(*fb, h_fb, 1, ops.S);
-    } else {
-        k_true_residual<<<gs, kBlock, 0, s>>>(ops, solver != MPS_SOLVER_CG64 ? 1 : 0);
-    }
+    k_mx_finish<<<ops.grid_vec, kBlock, 0, s>>>(ops);
+    const cudaError_t fe = fallback_kernels(ops, *fb, 1, s);
     e = cudaStreamEndCapture(s, &captured);
+    if (fe != cudaSuccess) return fe;
     if (e != cudaSuccess) return e;
-    if (with_fb) {
-        cudaGraphNode_t fb_init;
-        e = sink_node(graph_, &fb_init);
-        if (e != cudaSuccess) return e;
-        cudaGraphNode_t fb_while;
-        cudaGraph_t fb_body;
-        e = add_while(graph_, &fb_init, h_fb, &fb_while, &fb_body);
-        if (e != cudaSuccess) return e;
-        e = cudaStreamBeginCaptureToGraph(s, fb_body, nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return e;
-        cg64_body(*fb, h_fb, 1, s);
-        e = cudaStreamEndCapture(s, &captured);
-        if (e != cudaSuccess) return e;
-        e = cudaStreamBeginCaptureToGraph(s, graph_, &fb_while, nullptr, 1,
-                                          cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return e;
-        k_fb_merge<<<1, 32, 0, s>>>(ops.S, fb->S);
-        k_true_residual<<<gs, kBlock, 0, s>>>(ops, 1);
-        e = cudaStreamEndCapture(s, &captured);
-        if (e != cudaSuccess) return e;
-    }
 
     e = cudaGraphInstantiate(&exec_, graph_, 0);
     if (e != cudaSuccess) {
@@ -1629,11 +1575,7 @@ cudaError_t CgGraph::build_persistent(int solver, const CgOperands& ops, cudaStr
     persistent_ = true;
     kpi_ = 0;
     kri_ = 0;
-    const int gs = ops.grid_spmv;
     cudaError_t e = cudaGraphCreate(&graph_, 0);
-    if (e != cudaSuccess) return e;
-    cudaGraphConditionalHandle h_fb;
-    e = cudaGraphConditionalHandleCreate(&h_fb, graph_, 0, cudaGraphCondAssignDefault);
     if (e != cudaSuccess) return e;
     cudaGraph_t captured = nullptr;
     e = cudaStreamBeginCaptureToGraph(s, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
@@ -1655,26 +1597,9 @@ cudaError_t CgGraph::build_persistent(int solver, const CgOperands& ops, cudaStr
         GridSync g{ps.count, ps.gen, ps.err, ps.limits};
         cudaLaunchKernelEx(&cfg, k_pcg_persistent, ops, *mg, g);
     }
-    k_cg_init<<<gs, kBlock, 0, s>>>(*fb, h_fb, 1, ops.S);
+    const cudaError_t fe = fallback_kernels(ops, *fb, 0, s);  // the persistent loop records no true residual
     e = cudaStreamEndCapture(s, &captured);
-    if (e != cudaSuccess) return e;
-    cudaGraphNode_t fb_init;
-    e = sink_node(graph_, &fb_init);
-    if (e != cudaSuccess) return e;
-    cudaGraphNode_t fb_while;
-    cudaGraph_t fb_body;
-    e = add_while(graph_, &fb_init, h_fb, &fb_while, &fb_body);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamBeginCaptureToGraph(s, fb_body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
-    cg64_body(*fb, h_fb, 1, s);
-    e = cudaStreamEndCapture(s, &captured);
-    if (e != cudaSuccess) return e;
-    e = cudaStreamBeginCaptureToGraph(s, graph_, &fb_while, nullptr, 1, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
-    k_fb_merge<<<1, 32, 0, s>>>(ops.S, fb->S);
-    k_true_residual<<<gs, kBlock, 0, s>>>(ops, 0);  // the persistent loop does not record it
-    e = cudaStreamEndCapture(s, &captured);
+    if (fe != cudaSuccess) return fe;
     if (e != cudaSuccess) return e;
     e = cudaGraphInstantiate(&exec_, graph_, 0);
     if (e != cudaSuccess) {
@@ -1719,7 +1644,7 @@ cudaError_t host_loop(int solver, const CgOperands& ops, const MgHierarchy* mg, 
         for (int c = 0; c < chunk; c++) {
             body_kernels(solver, ops, mg, none, none, 0, true, s);
             // every kernel of the iteration and of the reliable update is launched
-            *k += cg_kernels_per_iteration(solver, mg) + cg_kernels_per_update(solver, mg, ops);
+            *k += cg_kernels_per_iteration(solver, mg) + cg_kernels_per_update(solver, mg);
         }
         e = cudaGetLastError();
     }
@@ -1745,7 +1670,7 @@ cudaError_t cg_run_direct(int solver, const CgOperands& ops, CgScalars* host_S, 
         k++;
     }
     if (solver != MPS_SOLVER_CG64 && fb) {
-        k_cg_init<<<gs, kBlock, 0, s>>>(*fb, none, 0, ops.S);
+        k_cg_init<<<gs, kBlock, 0, s>>>(*fb, ops.S);
         k++;
         e = host_loop(MPS_SOLVER_CG64, *fb, nullptr, host_S, chunk, s, &k);
         if (e != cudaSuccess) return e;

@@ -68,6 +68,8 @@ struct CgOperands {
     float* u32;         // preconditioned residual u = M r (MIXED_MG, LEARNED)
     double* partials;   // reduction partials (cg_partials doubles)
     uint32_t* tickets;  // per-group reduction counters (cg_tickets, zero between kernels)
+    double* slots;      // exchange words of the single-launch loops (kLoopSlots)
+    int32_t* loop_w;    // per chunk: its width, 0 when the loops leave it out (written by init)
     CgScalars* S;
     const DevStatus* status;  // step status (may be null): a failed search aborts the solve
 };
@@ -189,6 +191,17 @@ __device__ __forceinline__ float row32(const CgOperands& o, int64_t at, int L, c
 struct MgHierarchy;
 struct LearnedOps;
 
+// Iterations the plain mixed solver may run without a reliable update (a tenfold drop of
+// its recursive residual norm takes a few hundred iterations on the PPEs of the
+// workloads when the FP32 recursion makes progress).
+constexpr int kMixedStallIter = 2000;
+
+// cgloop.cu: the iteration loops of MPS_SOLVER_CG64 (after k_cg_init) and MPS_SOLVER_MIXED
+// (after k_mx_init and the first k_mx_spmv), one cooperative launch each.
+cudaError_t launch_cg_loop(const CgOperands& o, cudaStream_t s);
+cudaError_t launch_mx_loop(const CgOperands& o, cudaStream_t s);
+cudaError_t cg_loop_prepare_device();
+
 // Bounds of the device-side waits, in SM clock cycles, kept in device memory per handle
 // so that captured graphs read the current values.  A wait gives up once this many
 // cycles have passed since it began (0: at its first check), sets an error word and
@@ -220,8 +233,9 @@ struct LearnedRun {
     CgScalars* S;
 };
 
-// A CUDA graph running one whole solve: init kernels + device-driven while loop (+ for
-// the preconditioned solvers the FP64 CG fallback loop, which runs only after a failure).
+// A CUDA graph running one whole solve: init kernels + the iteration loop (one launch for
+// the plain solvers, a device-driven while loop for the preconditioned ones) + for the
+// mixed-precision solvers the FP64 CG fallback loop, which runs only after a failure.
 // Side stream and events of a fork/join inside a captured graph.
 struct SetupFork {
     cudaStream_t side = nullptr;
@@ -232,7 +246,7 @@ class CgGraph {
 public:
     ~CgGraph();
     // `mg` and `fb` (operands of the FP64 fallback, own scalars) are required for
-    // MPS_SOLVER_MIXED_MG and MPS_SOLVER_LEARNED and ignored otherwise.
+    // MPS_SOLVER_MIXED_MG and MPS_SOLVER_LEARNED; MPS_SOLVER_MIXED takes `fb` alone.
     cudaError_t build(int solver, const CgOperands& ops, cudaStream_t s,
                       const MgHierarchy* mg = nullptr, const CgOperands* fb = nullptr,
                       const LearnedRun* lrn = nullptr);
@@ -251,6 +265,7 @@ public:
     bool nested() const { return nested_; }
 
 private:
+    cudaError_t build_plain(int solver, const CgOperands& ops, cudaStream_t s, const CgOperands* fb);
     cudaError_t build_impl(int solver, const CgOperands& ops, cudaStream_t s, bool nested,
                            const MgHierarchy* mg, const CgOperands* fb, const LearnedRun* lrn);
     cudaGraph_t graph_ = nullptr;
@@ -273,7 +288,7 @@ cudaError_t cg_run_direct(int solver, const CgOperands& ops, CgScalars* host_S, 
 int persistent_blocks();
 // Kernels of one iteration of the solver, and of one reliable update.
 int cg_kernels_per_iteration(int solver, const MgHierarchy* mg);
-int cg_kernels_per_update(int solver, const MgHierarchy* mg, const CgOperands& ops);
+int cg_kernels_per_update(int solver, const MgHierarchy* mg);
 
 // Sets eps / criterion / max_iter / delta for the next solve (stream-ordered).
 void launch_cg_configure(CgScalars* S, double eps, int criterion, int max_iter, double delta2,

@@ -18,6 +18,7 @@
 #include "batch.cuh"
 #include "learned.cuh"
 #include "common.cuh"
+#include "gridloop.cuh"
 
 using namespace mpsgb;
 
@@ -54,6 +55,8 @@ struct mps_handle {
     CgScalars* S = nullptr;
     double* partials = nullptr;
     uint32_t* tickets = nullptr;
+    double* slots = nullptr;
+    int32_t* loop_w = nullptr;
     double *r = nullptr, *p = nullptr, *Ap = nullptr, *x2 = nullptr;
     float *r32 = nullptr, *w32 = nullptr, *s32 = nullptr, *p32 = nullptr, *d32 = nullptr;
     float* u32 = nullptr;
@@ -389,6 +392,8 @@ void allocate(mps_handle* h, int64_t n, int64_t keep) {
     st.solve_ok = &h->S->converged;
     h->partials = dalloc<double>(h, cg_partials(n));
     h->tickets = dalloc<uint32_t>(h, cg_tickets(n));
+    h->slots = dalloc<double>(h, kLoopSlots);
+    h->loop_w = dalloc<int32_t>(h, nchunks);
     h->r = dalloc<double>(h, n);
     h->p = dalloc<double>(h, n);
     h->Ap = dalloc<double>(h, n);
@@ -582,6 +587,8 @@ CgOperands cg_operands(mps_handle* h) {
     o.u32 = h->u32;
     o.partials = h->partials;
     o.tickets = h->tickets;
+    o.slots = h->slots;
+    o.loop_w = h->loop_w;
     o.S = h->S;
     o.status = h->st.status;
     return o;
@@ -628,6 +635,12 @@ int default_max_iter(int32_t requested, int64_t n, int32_t solver) {
     return static_cast<int>(std::min<int64_t>(lim, 0x7fffffff));
 }
 
+// Kernels of a plain solve's graph: init (and MIXED's first SpMV), the loop, [finish], with
+// a fallback its init, loop and merge, the true residual.
+int plain_solve_launches(int solver, bool with_fb) {
+    return solver == MPS_SOLVER_CG64 ? 3 : 5 + (with_fb ? 3 : 0);
+}
+
 void after_launch(const char* what) { check(cudaGetLastError(), what); }
 
 // Reads the status block and converts device flags into the reference's errors.
@@ -665,25 +678,22 @@ void read_status(mps_handle* h, bool solve_done) {
         if (h->direct_launches >= 0) {
             launched(h, static_cast<int>(h->direct_launches));
         } else if (h->prm.solver == MPS_SOLVER_CG64) {
-            launched(h, 2 + 3 * S.iter);
-        } else {
+            launched(h, plain_solve_launches(MPS_SOLVER_CG64, false));
+        } else if (is_preconditioned(h->prm.solver)) {
             const int kpi = h->cg.kernels_per_iteration(), kpu = h->cg.kernels_per_update();
-            if (is_preconditioned(h->prm.solver)) {
-                const int own = S.iter - S.fb_iter;
-                // per-phase kernels and the finish kernel, or one persistent kernel
-                const int loop = h->cg.persistent() ? 1 : own * kpi + S.updates * kpu + 1;
-                launched(h, mg_setup_launches(h->mg) + 2 + mg_apply_launches(h->mg) + loop + 3 + 3 * S.fb_iter +
-                                (h->prm.solver == MPS_SOLVER_LEARNED ? 1 + learned_prep_launches(h->mg, true) : 0));
-            } else {
-                const int own = S.iter - S.fb_iter;
-                launched(h, 4 + own * kpi + S.updates * kpu + (S.fallback ? 2 + 3 * S.fb_iter : 1));
-            }
+            const int own = S.iter - S.fb_iter;
+            // per-phase kernels and the finish kernel, or one persistent kernel
+            const int loop = h->cg.persistent() ? 1 : own * kpi + S.updates * kpu + 1;
+            launched(h, mg_setup_launches(h->mg) + 2 + mg_apply_launches(h->mg) + loop + 4 +
+                            (h->prm.solver == MPS_SOLVER_LEARNED ? 1 + learned_prep_launches(h->mg, true) : 0));
+        } else {
+            launched(h, plain_solve_launches(h->prm.solver, true));
         }
     }
     const int f = h->h_status->flags;
     if (f & kStatusCellOverflow) throw StatusError{MPS_ERR_CELL_OVERFLOW, "Too many particle in a block"};
     if (f & kStatusWaitTimeout)
-        throw StatusError{MPS_ERR_TIMEOUT, "a shared-memory stage of the SpMV stream timed out"};
+        throw StatusError{MPS_ERR_TIMEOUT, "a bounded wait of the solve timed out"};
     if (f & kStatusDeviceCheck) {
         char buf[96];
         std::snprintf(buf, sizeof(buf), "device bounds check fired at particle %d",
@@ -1956,6 +1966,8 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         o.d32 = loc.get<float>(nn);
         o.partials = loc.get<double>(static_cast<size_t>(cg_partials(n)));
         o.tickets = loc.get<uint32_t>(static_cast<size_t>(cg_tickets(n)));
+        o.slots = loc.get<double>(kLoopSlots);
+        o.loop_w = loc.get<int32_t>(static_cast<size_t>(nchunks));
         o.S = loc.get<CgScalars>(1);
         cudaStream_t s = h->stream;
         check(cudaMemsetAsync(o.tickets, 0, sizeof(uint32_t) * cg_tickets(n), s), "memset");
@@ -1974,6 +1986,7 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         check(cudaMemsetAsync(o.d32, 0, sizeof(float) * nn, s), "memset");
         check(cudaMemsetAsync(o.p32, 0, sizeof(float) * nn, s), "memset");
         launch_cg_configure(o.S, eps, criterion, default_max_iter(max_iters, n, solver), 0.01, s);
+        check(cg_prepare_device(), "solver kernel attributes");
         CgGraph g;
         check(g.build(solver, o, s), "CG graph build");
         check(g.launch(s), "CG graph launch");
@@ -1983,7 +1996,7 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         check(cudaStreamSynchronize(s), "cg solve");
         if (iterations) *iterations = S.iter;
         if (true_relres) *true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
-        h->stats.kernel_launches += 4 + S.iter * g.kernels_per_iteration() + 2 * S.updates;
+        h->stats.kernel_launches += 1 + plain_solve_launches(solver, false);
         if (!S.converged)
             throw StatusError{MPS_ERR_CG_NOT_CONVERGED,
                               "Conjugate Gradient method couldn't solve Pressure Poison Equation"};

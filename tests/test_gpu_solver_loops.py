@@ -1,0 +1,100 @@
+"""The plain solvers' single-launch loops at the edges of their work split.
+
+mps_cg_solve_csr runs the loop kernels on a caller's system, so the systems here choose the
+sizes: rows around a chunk (32), around the largest system one cluster takes (80 and 128
+chunks), several tiles of chunks per block, more chunks than a block's tables hold, rows
+longer than the usual unit, and identity rows (left out of the loop when their residual is
+zero, kept when it is not).
+
+Tolerance: each system is symmetric and strictly diagonally dominant with off-diagonal row
+sums of at most half the diagonal, so its condition number is at most 3 d_max / d_min <= 6,
+and |b - A x| <= 1e-12 |b| leaves |x - x*| <= 6e-12 |x*|; b = A x* adds rounding of 1e-15.
+"""
+import numpy as np
+import pytest
+
+from openmps_gb300 import _abi as abi
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-11
+
+
+def _system(n, offsets, seed, identity=0.0, dense_row=False):
+    """CSR of a banded symmetric system, x* and a starting guess."""
+    rng = np.random.default_rng(seed)
+    idn = rng.random(n) < identity
+    rows, cols, vals = [], [], []
+    for k in offsets:
+        if k >= n:
+            continue
+        i = np.arange(n - k)
+        i = i[~idn[i] & ~idn[i + k]]
+        v = rng.uniform(0.1, 1.0, i.size)
+        rows += [i, i + k]
+        cols += [i + k, i]
+        vals += [v, v]
+    if dense_row and n > 2:
+        j = np.arange(1, n)
+        j = j[~idn[j] & ~idn[0]]
+        v = rng.uniform(0.1, 1.0, j.size)
+        rows += [np.zeros(j.size, np.int64), j]
+        cols += [j, np.zeros(j.size, np.int64)]
+        vals += [v, v]
+    row = np.concatenate(rows) if rows else np.zeros(0, np.int64)
+    col = np.concatenate(cols) if cols else np.zeros(0, np.int64)
+    val = np.concatenate(vals) if vals else np.zeros(0)
+    # scaled so that no row's off-diagonal sum passes half of the diagonal 1 .. 2
+    total = np.bincount(row, weights=val, minlength=n)
+    val = val * (0.5 / max(total.max(), 1e-300)) if row.size else val
+    diag = np.where(idn, 1.0, rng.uniform(1.0, 2.0, n))
+    row = np.concatenate([row, np.arange(n)])
+    col = np.concatenate([col, np.arange(n)])
+    val = np.concatenate([val, diag])
+    order = np.lexsort((col, row))
+    row, col, val = row[order], col[order], val[order]
+    ptr = np.zeros(n + 1, np.int64)
+    ptr[1:] = np.cumsum(np.bincount(row, minlength=n))
+    xs = rng.standard_normal(n)
+    b = np.add.reduceat(val * xs[col], ptr[:-1])
+    x0 = xs + rng.standard_normal(n)
+    still = idn & (rng.random(n) < 0.5)  # identity rows that start at their solution
+    if identity > 0:
+        still |= idn & (np.arange(n) // 32 % 2 == 0)
+    x0[still] = b[still]
+    return ptr, col.astype(np.int32), val, b, xs, x0
+
+
+CASES = {
+    "one_row": dict(n=1, offsets=()),
+    "below_chunk": dict(n=31, offsets=(1,)),
+    "chunk": dict(n=32, offsets=(1, 7)),
+    "above_chunk": dict(n=33, offsets=(1, 7)),
+    "cluster64_edge": dict(n=80 * 32, offsets=(1, 2, 50, 51, 52)),
+    "cluster64_past": dict(n=80 * 32 + 1, offsets=(1, 2, 50, 51, 52)),
+    "cluster32_edge": dict(n=128 * 32, offsets=(1, 2, 64, 65)),
+    "cluster32_past": dict(n=128 * 32 + 1, offsets=(1, 2, 64, 65)),
+    "identity_rows": dict(n=5000, offsets=(1, 2, 3, 70, 71, 72), identity=0.7),
+    "all_but_identity": dict(n=20000, offsets=(1,), identity=0.98),
+    "long_row": dict(n=700, offsets=(1, 2), dense_row=True),
+    "wide_rows": dict(n=9000, offsets=tuple(range(1, 46))),
+    "two_tiles": dict(n=152 * 32 * 45 + 5, offsets=(1, 500)),
+    "tables_rebuilt": dict(n=1_700_001, offsets=(1,)),
+}
+
+
+@pytest.mark.parametrize("solver", ["cg64", "mixed"])
+@pytest.mark.parametrize("name", list(CASES))
+def test_loop_sizes(gpu_lib, name, solver):
+    from openmps_gb300.computer import Computer
+
+    ptr, col, val, b, xs, x0 = _system(seed=len(name), **CASES[name])
+    c = Computer(abi.make_params())
+    which = abi.SOLVER_CG64 if solver == "cg64" else abi.SOLVER_MIXED
+    x, it, rel = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    err = float(np.linalg.norm(x - xs) / np.linalg.norm(xs))
+    print("%s %s: n %d, %d iterations, relres %.2e, error %.2e" % (name, solver, len(b), it, rel, err))
+    assert rel <= 1.01e-12
+    assert err <= TOL
+    again, it2, _ = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    assert it2 == it and np.array_equal(x, again)  # every sum has a fixed order
