@@ -9,7 +9,7 @@
 // their CSR system in their own device buffers and need a solve that allocates
 // nothing.  This file provides that solve: the reference's FP64 CG
 // (Computer::SolvePressurePoissonEquation, src/OpenMps/Computer.hpp:1359-1429) whose
-// scratch vectors r, p, Ap, block partials and scalars live in one file-scope static
+// scratch vectors r, p, s, exchange words and scalars live in one file-scope static
 // device array of fixed size (kNoallocMaxRows rows).  Every GPU that loads the library
 // holds that array until the process exits.
 //
@@ -24,210 +24,280 @@
 // call's contents; the parts that must start at zero are cleared at the start of each
 // call.  Calls that overlap on the GPU (different streams or host threads at the same
 // time) race on the array.
+//
+// A call is one launch: initial residual, iterations and the final true residual in one
+// cluster of 16 blocks (small systems) or a cooperative grid of one block per SM, with the
+// two exchanges per iteration of gridloop.cuh and the recurrence of cgloop.cu (s = A r +
+// beta s).  Blocks own contiguous rows of equal entries; a few lanes share a row so that a
+// warp reads consecutive entries of the CSR arrays, and their partial sums meet in a
+// transposing exchange (four rows a lane, three additions instead of eight: the FP64 pipe
+// takes a warp-wide addition every 64 cycles).  Before, one thread walked a row (a warp's
+// loads touched 32 rows apart) in three kernels per iteration, and the host read the
+// convergence flag every 16 iterations.
 #include <cmath>
 
-#include "common.cuh"
+#include "gridloop.cuh"
 
 namespace mpsgb {
 
 namespace {
 
 constexpr int64_t kNoallocMaxRows = MPS_NOALLOC_MAX_ROWS;
-constexpr int kNoallocMaxBlocks = static_cast<int>((kNoallocMaxRows + kBlock - 1) / kBlock);
 constexpr int kNoallocScalars = 16;  // doubles reserved for NoallocScalars
-constexpr int64_t kNoallocDoubles = 3 * kNoallocMaxRows + 2 * kNoallocMaxBlocks + kNoallocScalars;
+constexpr int64_t kNoallocDoubles = 3 * kNoallocMaxRows + kLoopSlots + kNoallocScalars;
+// Rows up to which one cluster solves the system.  us per iteration on lattice operators,
+// before and now: 500 rows of 13 entries 23.1 -> 5.5 and 2,000 of 48 30.9 -> 8.9 (cluster);
+// 3,600 of 13 22.4 -> 7.7, 10,000 of 28 25.7 -> 9.5, 100,441 of 5 / 28 / 48 21.5 -> 10.3,
+// 31.1 -> 17.9 and 44.1 -> 24.0 (grid: two exchanges of about 3 us, then the FP64 pipe, 5.3
+// us at 28 entries).
+constexpr int64_t kNoallocClusterRows = 2048;
 
 struct NoallocScalars {
-    double rr, rr_new, alpha, beta, thr, bb, rr0, true_rr;
-    unsigned int counter;
-    int iter, converged, max_iter;
+    double bb, true_rr;
+    int iter, converged, timed_out, pad;
 };
 static_assert(sizeof(NoallocScalars) <= kNoallocScalars * sizeof(double), "scalars do not fit");
 
-// The solver's whole scratch: r, p, Ap, partials, scalars.
+// The solver's whole scratch: r, p, s, exchange words, scalars.
 static __device__ __align__(256) double g_noalloc_scratch[kNoallocDoubles];
 
-struct Scratch {
-    double *r, *p, *Ap, *partials;
+struct CsrSystem {
+    int n;
+    const int64_t* rp;
+    const int32_t* col;
+    const double* val;
+    const double* b;
+    double* x;
+    double *r, *p, *s, *slots;  // scratch
     NoallocScalars* S;
+    double eps;
+    int criterion, max_iter;
+    int keep_rows;  // rows whose vectors fit the block's shared memory
 };
 
-__device__ __forceinline__ Scratch carve(double* base, int64_t n) {
-    (void)n;
-    Scratch s;
-    s.r = base;
-    s.p = base + kNoallocMaxRows;
-    s.Ap = base + 2 * kNoallocMaxRows;
-    s.partials = base + 3 * kNoallocMaxRows;
-    s.S = reinterpret_cast<NoallocScalars*>(base + 3 * kNoallocMaxRows + 2 * kNoallocMaxBlocks);
-    return s;
+// How a block's warps walk its rows: LANES lanes share a row, GROUPS row groups of a warp at
+// once.  Lane per row for short rows, four lanes in transposing groups of four for ordinary
+// ones, fewer rows a warp when the block has few, a warp per row for long ones.
+enum RowWalk { kLanePerRow, kFourByFour, kFourLanes, kEightLanes, kWarpPerRow };
+
+__device__ __forceinline__ int walk_rows(int walk) {  // rows a warp takes at once
+    return walk == kLanePerRow || walk == kFourByFour ? 32 : walk == kFourLanes ? 8 : walk == kEightLanes ? 4 : 1;
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ double block_sum(double v, double* ws) {
-    ws[threadIdx.x] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x < 32) {
-        for (int k = threadIdx.x; k < static_cast<int>(blockDim.x); k += 32) s += ws[k];
-        s = warp_sum(s);
-    }
-    __syncthreads();
-    return s;
-}
-
-// Block partials s0, s1; true in the last block to finish (atomic ticket, no waiting).
-__device__ bool publish(double s0, double s1, const Scratch& sc) {
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        sc.partials[blockIdx.x] = s0;
-        sc.partials[gridDim.x + blockIdx.x] = s1;
-        __threadfence();
-        last = atomicAdd(&sc.S->counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    return last;
-}
-
-__device__ double gather(const double* partials, double* ws) {
-    double v = 0.0;
-    for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += blockDim.x) v += __ldcg(partials + k);
-    return block_sum(v, ws);
-}
-
-__device__ __forceinline__ double csr_row(int64_t i, const int64_t* rp, const int32_t* col,
-                                          const double* val, const double* v) {
-    double s = 0.0;
-    for (int64_t k = rp[i]; k < rp[i + 1]; k++) s = fma(val[k], v[col[k]], s);
-    return s;
-}
-
-// r = b - A x; p = r; rr, bb; threshold (Computer.hpp:1382-1389)
-__global__ void k_na_init(double* base, int64_t n, const int64_t* rp, const int32_t* col,
-                          const double* val, const double* b, const double* x, double eps,
-                          int criterion, int max_iter) {
-    __shared__ double ws[kBlock];
-    const Scratch sc = carve(base, n);
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    double vr = 0.0, vb = 0.0;
-    if (i < n) {
-        const double bi = b[i];
-        const double ri = bi - csr_row(i, rp, col, val, x);
-        sc.r[i] = ri;
-        sc.p[i] = ri;
-        vr = ri * ri;
-        vb = bi * bi;
-    }
-    const double s0 = block_sum(vr, ws);
-    const double s1 = block_sum(vb, ws);
-    if (publish(s0, s1, sc)) {
-        const double rr = gather(sc.partials, ws);
-        const double bb = gather(sc.partials + gridDim.x, ws);
-        if (threadIdx.x == 0) {
-            NoallocScalars* S = sc.S;
-            S->counter = 0;
-            S->rr = rr;
-            S->rr0 = rr;
-            S->rr_new = rr;
-            S->bb = bb;
-            double thr = rr * eps * eps;
-            if (criterion == MPS_CRIT_RHS && bb > 0) thr = bb * eps * eps;
-            S->thr = thr;
-            S->converged = (criterion == MPS_CRIT_RHS) ? ((rr < thr) || (rr == 0)) : (thr == 0);
-            S->iter = 0;
-            S->max_iter = max_iter;
+// f(row, (A v)_row) for rows [r0, r1), each in one lane
+template <int LANES, int GROUPS, class F>
+__device__ __forceinline__ void row_products(const CsrSystem& A, int r0, int r1, const double* v, F f) {
+    static_assert(GROUPS == 1 || GROUPS == LANES, "the exchange transposes a square");
+    constexpr int kPer = 32 / LANES;              // rows of a group
+    constexpr int kDepth = GROUPS > 1 ? 2 : 8 / (LANES >= 8 ? 2 : 1);  // entries of a row a lane loads at once
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = static_cast<int>(blockDim.x >> 5);
+    const int sub = lane % LANES, who = lane / LANES;
+    for (int base = r0 + warp * kPer * GROUPS; base < r1; base += warps * kPer * GROUPS) {
+        int64_t at[GROUPS];
+        int left[GROUPS];
+        double acc[GROUPS];
+        int most = 0;
+#pragma unroll
+        for (int g = 0; g < GROUPS; g++) {
+            const int row = base + g * kPer + who;
+            const int64_t b = row < r1 ? A.rp[row] : 0, e = row < r1 ? A.rp[row + 1] : 0;
+            at[g] = b + sub;
+            left[g] = static_cast<int>(e - b) - sub;  // > 0: entries from this lane's on
+            most = max(most, static_cast<int>(e - b));
+            acc[g] = 0.0;
         }
-    }
-}
-
-__device__ __forceinline__ bool na_done(const NoallocScalars* S) {
-    return S->converged || S->iter >= S->max_iter;
-}
-
-// Ap = A p; alpha = rr / p.Ap
-__global__ void k_na_spmv_dot(double* base, int64_t n, const int64_t* rp, const int32_t* col,
-                              const double* val) {
-    __shared__ double ws[kBlock];
-    const Scratch sc = carve(base, n);
-    if (na_done(sc.S)) return;
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    double v = 0.0;
-    if (i < n) {
-        const double s = csr_row(i, rp, col, val, sc.p);
-        sc.Ap[i] = s;
-        v = sc.p[i] * s;
-    }
-    const double s0 = block_sum(v, ws);
-    if (publish(s0, 0.0, sc)) {
-        const double pap = gather(sc.partials, ws);
-        if (threadIdx.x == 0) {
-            sc.S->counter = 0;
-            sc.S->alpha = sc.S->rr / pap;
-        }
-    }
-}
-
-// x += alpha p; r -= alpha Ap; rrNew; convergence; beta (Computer.hpp:1402-1420)
-__global__ void k_na_update(double* base, int64_t n, double* x) {
-    __shared__ double ws[kBlock];
-    const Scratch sc = carve(base, n);
-    if (na_done(sc.S)) return;
-    const double alpha = sc.S->alpha;
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    double v = 0.0;
-    if (i < n) {
-        x[i] = fma(alpha, sc.p[i], x[i]);
-        const double ri = fma(-alpha, sc.Ap[i], sc.r[i]);
-        sc.r[i] = ri;
-        v = ri * ri;
-    }
-    const double s0 = block_sum(v, ws);
-    if (publish(s0, 0.0, sc)) {
-        const double rr_new = gather(sc.partials, ws);
-        if (threadIdx.x == 0) {
-            NoallocScalars* S = sc.S;
-            S->counter = 0;
-            S->rr_new = rr_new;
-            S->converged = rr_new < S->thr;
-            if (!S->converged) {
-                S->beta = rr_new / S->rr;
-                S->rr = rr_new;
+        most = __reduce_max_sync(0xffffffffu, most);
+        for (int k = 0; k < most; k += kDepth * LANES) {
+            int c[GROUPS][kDepth];
+            double a[GROUPS][kDepth];
+#pragma unroll
+            for (int g = 0; g < GROUPS; g++) {
+#pragma unroll
+                for (int d = 0; d < kDepth; d++) {
+                    const bool in = k + d * LANES < left[g];
+                    c[g][d] = in ? __ldg(A.col + at[g] + k + d * LANES) : 0;
+                    a[g][d] = in ? __ldg(A.val + at[g] + k + d * LANES) : 0.0;
+                }
             }
-            S->iter += 1;
+            double xv[GROUPS][kDepth];
+#pragma unroll
+            for (int g = 0; g < GROUPS; g++) {
+#pragma unroll
+                for (int d = 0; d < kDepth; d++) xv[g][d] = k + d * LANES < left[g] ? v[c[g][d]] : 0.0;
+            }
+#pragma unroll
+            for (int d = 0; d < kDepth; d++) {
+#pragma unroll
+                for (int g = 0; g < GROUPS; g++)
+                    if (k + d * LANES < left[g]) acc[g] = fma(a[g][d], xv[g][d], acc[g]);
+            }
+        }
+        if constexpr (GROUPS == 4) {
+            // lane `sub` of four ends with the row of group `sub`
+            const bool hi = (sub & 2) != 0, odd = (sub & 1) != 0;
+            const double m0 = hi ? acc[2] : acc[0], m1 = hi ? acc[3] : acc[1];
+            const double o0 = hi ? acc[0] : acc[2], o1 = hi ? acc[1] : acc[3];
+            const double t0 = m0 + __shfl_xor_sync(0xffffffffu, o0, 2), t1 = m1 + __shfl_xor_sync(0xffffffffu, o1, 2);
+            const double mine = odd ? t1 : t0, other = odd ? t0 : t1;
+            const double sum = mine + __shfl_xor_sync(0xffffffffu, other, 1);
+            const int row = base + sub * kPer + who;
+            if (row < r1) f(row, sum);
+        } else {
+            double sum = acc[0];
+#pragma unroll
+            for (int o = LANES / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (sub == 0 && base + who < r1) f(base + who, sum);
         }
     }
 }
 
-// p = r + beta p
-__global__ void k_na_pupdate(double* base, int64_t n) {
-    const Scratch sc = carve(base, n);
-    if (na_done(sc.S)) return;
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i < n) sc.p[i] = fma(sc.S->beta, sc.p[i], sc.r[i]);
+template <class F>
+__device__ __forceinline__ void csr_product(const CsrSystem& A, int walk, int r0, int r1, const double* v, F f) {
+    switch (walk) {
+        case kLanePerRow: row_products<1, 1>(A, r0, r1, v, f); break;
+        case kFourByFour: row_products<4, 4>(A, r0, r1, v, f); break;
+        case kFourLanes: row_products<4, 1>(A, r0, r1, v, f); break;
+        case kEightLanes: row_products<8, 1>(A, r0, r1, v, f); break;
+        default: row_products<32, 1>(A, r0, r1, v, f); break;
+    }
 }
 
-// |b - A x|^2 into S->true_rr
-__global__ void k_na_true(double* base, int64_t n, const int64_t* rp, const int32_t* col,
-                          const double* val, const double* b, const double* x) {
-    __shared__ double ws[kBlock];
-    const Scratch sc = carve(base, n);
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    double v = 0.0;
-    if (i < n) {
-        const double ri = b[i] - csr_row(i, rp, col, val, x);
-        v = ri * ri;
+// The first row i with (entries before it) + a i >= share (rows 0 .. n).
+__device__ __forceinline__ int row_at(const CsrSystem& A, int64_t a, int64_t share) {
+    int lo = 0, hi = A.n;
+    const int64_t first = A.rp[0];
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (A.rp[mid] - first + a * mid < share) lo = mid + 1;
+        else hi = mid;
     }
-    const double s0 = block_sum(v, ws);
-    if (publish(s0, 0.0, sc)) {
-        const double rr = gather(sc.partials, ws);
-        if (threadIdx.x == 0) {
-            sc.S->counter = 0;
-            sc.S->true_rr = rr;
+    return lo;
+}
+
+template <bool kCluster>
+__global__ void __launch_bounds__(kLoopThreads, 1) k_na_solve(CsrSystem A) {
+    extern __shared__ __align__(16) double na_sm[];
+    __shared__ LoopReduce red;
+    __shared__ struct {
+        double rr, alpha, beta, thr, bb, true_rr;
+        int iter, conv;
+    } sc;
+    __shared__ int range[2];
+    if (kCluster) loop_cluster_start();
+    LoopSync ls{A.slots, gridDim.x, 0};
+    const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
+    {
+        const int64_t nnz = A.rp[A.n] - A.rp[0];
+        const int64_t a = max(static_cast<int64_t>(1), nnz / (4 * static_cast<int64_t>(A.n)));
+        const int64_t total = nnz + a * A.n;
+        if (t < 2) range[t] = row_at(A, a, (blockIdx.x + t) * total / gridDim.x);
+    }
+    __syncthreads();
+    const int r0 = range[0], r1 = blockIdx.x + 1 == gridDim.x ? A.n : range[1], rows = r1 - r0;
+    const int64_t entries = A.rp[r1] - A.rp[r0];
+    const bool many = rows >= nt;
+    const int walk = entries > 128 * static_cast<int64_t>(rows) ? kWarpPerRow
+                     : many ? (entries <= 6 * static_cast<int64_t>(rows) ? kLanePerRow : kFourByFour)
+                            : (rows >= nt / 4 ? kFourLanes : kEightLanes);
+    const int warps_on = min(nt >> 5, (rows + walk_rows(walk) - 1) / walk_rows(walk));
+    const int product_lanes = 32 * warps_on, row_lanes = min(nt, rows);
+    // the block's rows of p, s, x and r, kept in shared memory when they fit
+    const bool keep = rows <= A.keep_rows;
+    double* P = keep ? na_sm - r0 : A.p;
+    double* Q = keep ? na_sm + rows - r0 : A.s;
+    double* X = keep ? na_sm + 2 * rows - r0 : A.x;
+    double* R = keep ? na_sm + 3 * rows - r0 : A.r;
+    bool ok;
+    {
+        // r = b - A x, p = s = 0, r.r, b.b, threshold (Computer.hpp:1382-1389)
+        double v[2] = {0.0, 0.0};
+        csr_product(A, walk, r0, r1, A.x, [&](int row, double ax) {
+            const double bi = A.b[row], ri = bi - ax;
+            P[row] = 0.0;
+            Q[row] = 0.0;
+            R[row] = ri;
+            if (keep) {
+                A.r[row] = ri;
+                X[row] = A.x[row];
+            }
+            v[0] = fma(ri, ri, v[0]);
+            v[1] = fma(bi, bi, v[1]);
+        });
+        ok = loop_reduce<kCluster, 2>(ls, red, v, product_lanes, [&](const double* tot) {
+            if (threadIdx.x != 0) return;
+            const double rr = tot[0], bb = tot[1];
+            double thr = rr * A.eps * A.eps;
+            if (A.criterion == MPS_CRIT_RHS && bb > 0) thr = bb * A.eps * A.eps;
+            sc.rr = rr;
+            sc.bb = bb;
+            sc.thr = thr;
+            sc.beta = 0.0;
+            sc.iter = 0;
+            sc.conv = A.criterion == MPS_CRIT_RHS ? (rr < thr || rr == 0) : thr == 0;
+        });
+    }
+    while (ok && !sc.conv && sc.iter < A.max_iter) {
+        // p = r + beta p; s = A r + beta s; alpha = r.r / p.s
+        double v = 0.0;
+        {
+            const double beta = sc.beta;
+            csr_product(A, walk, r0, r1, A.r, [&](int row, double ar) {
+                const double p = fma(beta, P[row], R[row]);
+                const double s = fma(beta, Q[row], ar);
+                P[row] = p;
+                Q[row] = s;
+                v = fma(p, s, v);
+            });
         }
+        ok = loop_reduce<kCluster, 1>(ls, red, &v, product_lanes, [&](const double* tot) {
+            const double alpha = ddiv_rn(sc.rr, tot[0]);
+            if (threadIdx.x == 0) sc.alpha = alpha;
+        });
+        if (!ok) break;
+        // x += alpha p; r -= alpha s; r.r; convergence; beta (Computer.hpp:1402-1420)
+        v = 0.0;
+        {
+            const double alpha = sc.alpha;
+            for (int row = r0 + t; row < r1; row += nt) {
+                X[row] = fma(alpha, P[row], X[row]);
+                const double ri = fma(-alpha, Q[row], R[row]);
+                R[row] = ri;
+                if (keep) A.r[row] = ri;
+                v = fma(ri, ri, v);
+            }
+        }
+        ok = loop_reduce<kCluster, 1>(ls, red, &v, row_lanes, [&](const double* tot) {
+            const double beta = ddiv_rn(tot[0], sc.rr);
+            __syncwarp();
+            if (threadIdx.x != 0) return;
+            sc.conv = tot[0] < sc.thr;
+            if (!sc.conv) {
+                sc.beta = beta;
+                sc.rr = tot[0];
+            }
+            sc.iter++;
+        });
+    }
+    // |b - A x|^2 of the x returned
+    if (keep)
+        for (int row = r0 + t; row < r1; row += nt) A.x[row] = X[row];
+    ok = ok && loop_reduce<kCluster, 0>(ls, red, nullptr, 0, [](const double*) {});
+    if (ok) {
+        double v = 0.0;
+        csr_product(A, walk, r0, r1, A.x, [&](int row, double ax) {
+            const double ri = A.b[row] - ax;
+            v = fma(ri, ri, v);
+        });
+        ok = loop_reduce<kCluster, 1>(ls, red, &v, product_lanes, [&](const double* tot) {
+            if (threadIdx.x == 0) sc.true_rr = tot[0];
+        });
+    }
+    if (blockIdx.x == 0 && t == 0) {
+        A.S->bb = sc.bb;
+        A.S->true_rr = sc.true_rr;
+        A.S->iter = sc.iter;
+        A.S->converged = ok ? sc.conv : 0;
+        A.S->timed_out = ok ? 0 : 1;
     }
 }
 
@@ -240,6 +310,49 @@ int scratch_for_current_context(double** out) {
     }
     *out = static_cast<double*>(ptr);
     return MPS_OK;
+}
+
+// One cluster for small systems, else a block per SM; p, s, x, r of half as many rows again
+// as the average block owns in shared memory.
+cudaError_t launch_na_solve(CsrSystem& A, cudaStream_t s) {
+    int dev = 0, sms = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    bool cluster = A.n <= kNoallocClusterRows;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.blockDim = dim3(kLoopThreads);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    for (;; cluster = false) {
+        auto kernel = cluster ? k_na_solve<true> : k_na_solve<false>;
+        const int blocks = cluster ? kLoopCluster : (sms < kLoopMaxBlocks ? sms : kLoopMaxBlocks);
+        const int64_t room = (most - 16 * 1024) / (4 * static_cast<int64_t>(sizeof(double)));
+        const int64_t want = 3 * static_cast<int64_t>(A.n) / (2 * blocks) + 128;
+        A.keep_rows = static_cast<int>(want < room ? want : room);
+        cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+        cfg.dynamicSmemBytes = static_cast<size_t>(A.keep_rows) * 4 * sizeof(double);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(cfg.dynamicSmemBytes));
+        if (e != cudaSuccess) return e;
+        if (!cluster) {
+            at[0].id = cudaLaunchAttributeCooperative;
+            at[0].val.cooperative = 1;
+            return cudaLaunchKernelEx(&cfg, kernel, A);
+        }
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kLoopCluster;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        int fit = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0)
+            return cudaLaunchKernelEx(&cfg, kernel, A);
+        cudaGetLastError();  // no cluster of this size: the grid
+    }
 }
 
 }  // namespace
@@ -260,31 +373,30 @@ extern "C" int mps_cg_solve_csr_device_noalloc(int64_t n, const int64_t* row_ptr
     const int rc = scratch_for_current_context(&base);
     if (rc != MPS_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int grid = static_cast<int>((n + kBlock - 1) / kBlock);
-    const int max_iter = max_iters > 0 ? max_iters : static_cast<int>(n);
-    // the ticket counter and the scalars start from zero on every call
-    double* scalars = base + 3 * kNoallocMaxRows + 2 * kNoallocMaxBlocks;
-    if (cudaMemsetAsync(scalars, 0, kNoallocScalars * sizeof(double), s) != cudaSuccess) return MPS_ERR_CUDA;
-    k_na_init<<<grid, kBlock, 0, s>>>(base, n, row_ptr, col, val, b, x, eps, criterion, max_iter);
+    CsrSystem A{};
+    A.n = static_cast<int>(n);
+    A.rp = row_ptr;
+    A.col = col;
+    A.val = val;
+    A.b = b;
+    A.x = x;
+    A.r = base;
+    A.p = base + kNoallocMaxRows;
+    A.s = base + 2 * kNoallocMaxRows;
+    A.slots = base + 3 * kNoallocMaxRows;
+    A.S = reinterpret_cast<NoallocScalars*>(A.slots + kLoopSlots);
+    A.eps = eps;
+    A.criterion = criterion;
+    A.max_iter = max_iters > 0 ? max_iters : static_cast<int>(n);
+    // the arrival counter starts from zero on every call
     NoallocScalars S{};
-    const int kCheck = 16;  // iterations between host reads of the convergence flag
-    for (;;) {
-        if (cudaGetLastError() != cudaSuccess) return MPS_ERR_CUDA;
-        if (cudaMemcpyAsync(&S, scalars, sizeof(S), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return MPS_ERR_CUDA;
-        if (S.converged || S.iter >= S.max_iter) break;
-        for (int c = 0; c < kCheck; c++) {
-            k_na_spmv_dot<<<grid, kBlock, 0, s>>>(base, n, row_ptr, col, val);
-            k_na_update<<<grid, kBlock, 0, s>>>(base, n, x);
-            k_na_pupdate<<<grid, kBlock, 0, s>>>(base, n);
-        }
-    }
-    k_na_true<<<grid, kBlock, 0, s>>>(base, n, row_ptr, col, val, b, x);
-    if (cudaGetLastError() != cudaSuccess ||
-        cudaMemcpyAsync(&S, scalars, sizeof(S), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
+    if (cudaMemsetAsync(A.slots, 0, sizeof(double), s) != cudaSuccess || launch_na_solve(A, s) != cudaSuccess ||
+        cudaMemcpyAsync(&S, A.S, sizeof(S), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess) {
+        cudaGetLastError();
         return MPS_ERR_CUDA;
+    }
+    if (S.timed_out) return MPS_ERR_TIMEOUT;
     if (iterations) *iterations = S.iter;
     if (true_relres) *true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
     return S.converged ? MPS_OK : MPS_ERR_CG_NOT_CONVERGED;

@@ -1,6 +1,6 @@
 """The plain solvers' single-launch loops at the edges of their work split.
 
-mps_cg_solve_csr runs the loop kernels on a caller's system, so the systems here choose the
+mps_cg_solve_csr and the allocation-free solve run on a caller's system, so the systems here choose the
 sizes: rows around a chunk (32), around the largest system one cluster takes (80 and 128
 chunks), several tiles of chunks per block, more chunks than a block's tables hold, rows
 longer than the usual unit, and identity rows (left out of the loop when their residual is
@@ -98,3 +98,44 @@ def test_loop_sizes(gpu_lib, name, solver):
     assert err <= TOL
     again, it2, _ = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
     assert it2 == it and np.array_equal(x, again)  # every sum has a fixed order
+
+
+# every way the allocation-free solve walks its rows, around the largest system one cluster
+# takes (2,048 rows) and at the largest it accepts
+NOALLOC = {
+    "one_row": dict(n=1, offsets=()),
+    "cluster_edge": dict(n=2048, offsets=(1, 2, 50, 51)),
+    "cluster_past": dict(n=2049, offsets=(1, 2, 50, 51)),
+    "eight_lanes": dict(n=5003, offsets=(1, 2, 70, 71, 72)),
+    "four_lanes": dict(n=30001, offsets=(1, 2, 3, 170, 171, 172)),
+    "four_by_four": dict(n=100_003, offsets=(1, 2, 3, 4, 315, 316, 317)),
+    "four_by_four_wide": dict(n=80_000, offsets=tuple(range(1, 24))),
+    "lane_per_row": dict(n=100_003, offsets=(1,)),
+    "warp_per_row": dict(n=2001, offsets=tuple(range(1, 100))),
+    "long_row": dict(n=700, offsets=(1, 2), dense_row=True),
+    "identity_rows": dict(n=20_000, offsets=(1, 2, 3), identity=0.9),
+    "largest": dict(n=abi.NOALLOC_MAX_ROWS, offsets=(1, 2, 512)),
+}
+
+
+@pytest.mark.parametrize("name", list(NOALLOC))
+def test_noalloc_sizes(gpu_lib, name):
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    ptr, col, val, b, xs, x0 = _system(seed=len(name), **NOALLOC[name])
+    dev = [torch.from_numpy(a).cuda() for a in (ptr, col, val, b)]
+    got = []
+    for _ in range(2):
+        x = torch.from_numpy(x0.copy()).cuda()
+        it, rel = C.c_int32(), C.c_double()
+        rc = gpu_lib.mps_cg_solve_csr_device_noalloc(len(b), *[a.data_ptr() for a in dev], x.data_ptr(), 1e-12,
+                                                     abi.CRIT_RHS, 0, torch.cuda.current_stream().cuda_stream,
+                                                     C.byref(it), C.byref(rel))
+        assert rc == abi.MPS_OK
+        got.append(x.cpu().numpy())
+    err = float(np.linalg.norm(got[0] - xs) / np.linalg.norm(xs))
+    print("%s: n %d, %d iterations, relres %.2e, error %.2e" % (name, len(b), it.value, rel.value, err))
+    assert rel.value <= 1.01e-12
+    assert err <= TOL
+    assert np.array_equal(got[0], got[1])
