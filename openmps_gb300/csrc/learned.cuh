@@ -98,21 +98,24 @@ void launch_learned_targets(const LearnedOps& L, const CgOperands& o, const CgSc
 cudaError_t mlp_prepare_device();
 
 // FP32 training: loss and gradient of `n` samples (partials per block, then summed in
-// a fixed order); Adam step.
+// a fixed order), and the same with the Adam step.
 struct MlpTrainer {
-    int64_t cap = 0;
-    float* samples = nullptr;   // cap x 18
-    float* w = nullptr;         // blob
-    float* m = nullptr;         // Adam moments (kMlpBlobFloats each)
+    const float* samples = nullptr;  // training set, rows of 18
+    float* w = nullptr;              // blob
+    float* m = nullptr;              // Adam moments (kMlpBlobFloats each)
     float* v = nullptr;
     float* grad = nullptr;      // kMlpBlobFloats
-    float* partials = nullptr;  // blocks x (kMlpParams + 1)
-    double* loss = nullptr;
-    int blocks_cap = 0;
+    float* partials = nullptr;  // mlp_train_partials x kMlpParams
+    float* losses = nullptr;    // of the samples of one call
+    double* loss = nullptr;     // their sum
 };
-int mlp_train_blocks(int64_t n);
+int mlp_train_partials(int64_t n);
 void launch_mlp_loss_grad(const MlpTrainer& T, const float* samples, int64_t n, cudaStream_t s);
-void launch_mlp_adam(const MlpTrainer& T, float lr, int step, cudaStream_t s);
+// pick[i] in [0, i], i = n - 1 .. 1: the draws of one epoch's Fisher-Yates shuffle.
+void launch_mlp_draws(uint64_t state, int64_t n, int64_t* pick, cudaStream_t s);
+// Adam step number `step` (from 1) on rows order[0 .. n - 1] of T.samples; *loss: their loss.
+void launch_mlp_train_step(const MlpTrainer& T, const int64_t* order, int64_t n, float lr, int step, double* loss,
+                           cudaStream_t s);
 cudaError_t mlp_train_prepare_device();
 
 }  // namespace mpsgb

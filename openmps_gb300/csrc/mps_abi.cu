@@ -1018,6 +1018,16 @@ struct ScopedBuffers {
     }
 };
 
+struct ScopedStream {
+    cudaStream_t s = nullptr;
+    ~ScopedStream() {
+        if (s) {
+            cudaStreamSynchronize(s);
+            cudaStreamDestroy(s);
+        }
+    }
+};
+
 // Runs f with `device` current, converting errors into status codes (standalone calls
 // that have no handle).
 template <class F>
@@ -2108,7 +2118,8 @@ int mps_mlp_loss_grad(int32_t device, const float* blob, const float* samples, i
         MlpTrainer T;
         T.w = b.get<float>(kMlpBlobFloats);
         T.grad = b.get<float>(kMlpBlobFloats);
-        T.partials = b.get<float>(static_cast<size_t>(mlp_train_blocks(n)) * (kMlpParams + 1));
+        T.partials = b.get<float>(static_cast<size_t>(mlp_train_partials(n)) * kMlpParams);
+        T.losses = b.get<float>(static_cast<size_t>(n));
         T.loss = b.get<double>(1);
         float* ds = b.get<float>(static_cast<size_t>(n) * kMlpSampleFloats);
         check(cudaMemcpy(T.w, blob, sizeof(float) * kMlpBlobFloats, cudaMemcpyHostToDevice), "copy");
@@ -2132,47 +2143,63 @@ int mps_mlp_train(int32_t device, float* blob, const float* samples, int64_t n, 
         ScopedBuffers b;
         MlpTrainer T;
         const int64_t bsz = std::min<int64_t>(batch, n);
+        const int64_t steps = (n + bsz - 1) / bsz;
         T.w = b.get<float>(kMlpBlobFloats);
         T.m = b.get<float>(kMlpBlobFloats);
         T.v = b.get<float>(kMlpBlobFloats);
-        T.grad = b.get<float>(kMlpBlobFloats);
-        T.partials = b.get<float>(static_cast<size_t>(mlp_train_blocks(bsz)) * (kMlpParams + 1));
-        T.loss = b.get<double>(1);
+        T.partials = b.get<float>(static_cast<size_t>(mlp_train_partials(bsz)) * kMlpParams);
+        T.losses = b.get<float>(static_cast<size_t>(bsz));
+        T.loss = b.get<double>(static_cast<size_t>(steps));
         float* ds = b.get<float>(static_cast<size_t>(n) * kMlpSampleFloats);
+        int64_t* order = b.get<int64_t>(static_cast<size_t>(n));
+        T.samples = ds;
+        // per epoch: a seeded Fisher-Yates shuffle of the samples (SplitMix64), then
+        // minibatches in order.  The draws are the device's (a 64-bit remainder each), on a
+        // stream of their own, the swaps the host's while the device works on the epoch
+        // before, and the device reads the samples through the permutation.
+        int64_t* pick = b.get<int64_t>(static_cast<size_t>(n));
+        std::vector<int64_t> perm(static_cast<size_t>(n)), host_pick(static_cast<size_t>(n));
+        ScopedStream draws;
+        check(cudaStreamCreateWithFlags(&draws.s, cudaStreamNonBlocking), "stream");
+        uint64_t state = seed;
+        auto draw = [&] {
+            launch_mlp_draws(state, n, pick, draws.s);
+            check(cudaGetLastError(), "shuffle draws");
+            state += static_cast<uint64_t>(n - 1) * 0x9e3779b97f4a7c15ull;
+        };
+        auto shuffle = [&] {
+            if (n > 1)
+                check(cudaMemcpyAsync(host_pick.data() + 1, pick + 1, sizeof(int64_t) * static_cast<size_t>(n - 1),
+                                      cudaMemcpyDeviceToHost, draws.s),
+                      "copy");
+            check(cudaStreamSynchronize(draws.s), "shuffle draws");
+            for (int64_t i = 0; i < n; i++) perm[i] = i;
+            for (int64_t i = n - 1; i > 0; i--) std::swap(perm[i], perm[host_pick[i]]);
+        };
+        draw();
         check(cudaMemcpy(T.w, blob, sizeof(float) * kMlpBlobFloats, cudaMemcpyHostToDevice), "copy");
         check(cudaMemset(T.m, 0, sizeof(float) * kMlpBlobFloats), "memset");
         check(cudaMemset(T.v, 0, sizeof(float) * kMlpBlobFloats), "memset");
-        check(cudaMemset(T.grad, 0, sizeof(float) * kMlpBlobFloats), "memset");
-        // per epoch: a seeded Fisher-Yates shuffle of the samples (SplitMix64), then
-        // minibatches in order
-        std::vector<float> shuffled(static_cast<size_t>(n) * kMlpSampleFloats);
-        std::vector<int64_t> perm(static_cast<size_t>(n));
-        uint64_t state = seed;
-        auto next = [&state]() {
-            uint64_t z = (state += 0x9e3779b97f4a7c15ull);
-            z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-            z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-            return z ^ (z >> 31);
+        check(cudaMemcpy(ds, samples, sizeof(float) * kMlpSampleFloats * n, cudaMemcpyHostToDevice), "copy");
+        std::vector<double> losses(static_cast<size_t>(steps));
+        auto collect = [&](int ep) {  // waits for the epoch
+            check(cudaMemcpy(losses.data(), T.loss, sizeof(double) * losses.size(), cudaMemcpyDeviceToHost), "copy");
+            double total = 0.0;
+            for (double l : losses) total += l;
+            if (epoch_loss) epoch_loss[ep] = total / static_cast<double>(n);
         };
         int step = 0;
+        shuffle();
         for (int ep = 0; ep < epochs; ep++) {
-            for (int64_t i = 0; i < n; i++) perm[i] = i;
-            for (int64_t i = n - 1; i > 0; i--) std::swap(perm[i], perm[next() % static_cast<uint64_t>(i + 1)]);
-            for (int64_t i = 0; i < n; i++)
-                std::memcpy(&shuffled[i * kMlpSampleFloats], samples + perm[i] * kMlpSampleFloats,
-                            sizeof(float) * kMlpSampleFloats);
-            check(cudaMemcpy(ds, shuffled.data(), sizeof(float) * shuffled.size(), cudaMemcpyHostToDevice), "copy");
-            double total = 0.0;
-            for (int64_t at = 0; at < n; at += bsz) {
-                const int64_t cnt = std::min(bsz, n - at);
-                launch_mlp_loss_grad(T, ds + at * kMlpSampleFloats, cnt, 0);
-                launch_mlp_adam(T, lr, ++step, 0);
-                double l = 0.0;
-                check(cudaMemcpy(&l, T.loss, sizeof(double), cudaMemcpyDeviceToHost), "copy");
-                total += l;
-            }
+            check(cudaMemcpy(order, perm.data(), sizeof(int64_t) * perm.size(), cudaMemcpyHostToDevice), "copy");
+            for (int64_t at = 0; at < n; at += bsz)
+                launch_mlp_train_step(T, order + at, std::min(bsz, n - at), lr, ++step, T.loss + at / bsz, 0);
             check(cudaGetLastError(), "training kernels");
-            if (epoch_loss) epoch_loss[ep] = total / static_cast<double>(n);
+            if (ep + 1 < epochs) {
+                draw();
+                shuffle();
+            }
+            collect(ep);
         }
         check(cudaMemcpy(blob, T.w, sizeof(float) * kMlpBlobFloats, cudaMemcpyDeviceToHost), "copy");
     });

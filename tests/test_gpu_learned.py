@@ -40,6 +40,43 @@ def test_gradient_matches_oracle(gpu_lib, n):
     assert err < 1e-4, err
 
 
+@pytest.mark.parametrize("n,batch", [(1, 4), (31, 31), (33, 64), (64, 64), (130, 64), (5000, 4900)])
+def test_training_steps_match_oracle(gpu_lib, n, batch):
+    # Three epochs of the same minibatches in FP64 (the shuffle by SplitMix64 and Fisher-Yates).
+    # An entry moves by about lr a step whatever its gradient's size, so one whose gradient is
+    # at the FP32 sums' rounding (1e-6 of the largest) may move the other way: a few in a
+    # thousand of them, hence the bound of 2 % of the movement in the 2-norm.
+    blob, samples = _random_case(5 + n, n)
+    lr, epochs, seed = 1e-3, 3, 9
+    got, losses = mlp_train(blob, samples, epochs=epochs, batch=batch, lr=lr, seed=seed)
+    w = blob.astype(np.float64)
+    m, v = np.zeros_like(w), np.zeros_like(w)
+    mask = (1 << 64) - 1
+    state, step, expect = seed, 0, []
+    for _ in range(epochs):
+        perm = list(range(n))
+        for i in range(n - 1, 0, -1):
+            state = (state + 0x9E3779B97F4A7C15) & mask
+            z = ((state ^ (state >> 30)) * 0xBF58476D1CE4E5B9) & mask
+            z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & mask
+            j = (z ^ (z >> 31)) % (i + 1)
+            perm[i], perm[j] = perm[j], perm[i]
+        total = 0.0
+        for at in range(0, n, batch):
+            part = samples[perm[at:at + batch]].astype(np.float64)
+            loss, grad = mlp.loss_grad(w, part)
+            total += loss * len(part)
+            step += 1
+            m = 0.9 * m + 0.1 * grad
+            v = 0.999 * v + 0.001 * grad * grad
+            w = w - lr * (m / (1 - 0.9 ** step)) / (np.sqrt(v / (1 - 0.999 ** step)) + 1e-8)
+        expect.append(total / n)
+    assert np.array_equal(got[:32], blob[:32])
+    moved = lr * step * np.sqrt(w.size)
+    assert np.linalg.norm(got - w) <= 0.02 * moved
+    np.testing.assert_allclose(losses, expect, rtol=1e-3)
+
+
 @pytest.mark.parametrize("n", [1, 127, 128, 129, 20000])
 def test_tensor_core_inference_matches_oracle(gpu_lib, n):
     blob, samples = _random_case(7 + n, n)
