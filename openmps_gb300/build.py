@@ -33,6 +33,7 @@ UNITS = {
     "dim3.cu": ["-fmad=false"],
     "cg.cu": [],
     "cgloop.cu": [],
+    "pcgloop.cu": [],
     "mg.cu": [],
     "learned.cu": [],
     "batch.cu": [],

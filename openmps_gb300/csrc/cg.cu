@@ -1,10 +1,10 @@
 // cg.cu - pressure Poisson solvers (Computer::SolvePressurePoissonEquation,
 // Computer.hpp:1359-1429) on the SELL-32 matrix, each run as one CUDA graph: init kernels,
-// then the iterations: one launch for the plain solvers (cgloop.cu), a conditional WHILE node
-// whose body is a few kernels for the preconditioned ones; the last block of each reduction
-// decides the next step and sets the graph condition, so a solve of thousands of iterations
-// needs no host round trip.  With MPS_CG_LAUNCH_HOST every phase of every solver is launched
-// by the host.
+// then the iterations: one launch (cgloop.cu; pcgloop.cu where the hierarchy fits it), or for
+// the larger preconditioned systems a conditional WHILE node whose body is a few kernels; the
+// last block of each reduction decides the next step and sets the graph condition, so a solve
+// of thousands of iterations needs no host round trip.  MPS_CG_LAUNCH_HOST issues the same
+// kernels from the host.
 //
 // Work layout: vector kernels run one thread per row, SpMV kernels one warp per chunk of
 // 32 rows (one lane per row, as many warps as chunks, so the block scheduler balances
@@ -20,7 +20,7 @@
 // the group's, and the last group adds the group sums (atomic tickets, no waiting).  Every
 // addition has a fixed order, so results are deterministic run to run.
 //
-// MPS_SOLVER_CG64: the reference CG in FP64 (3 kernels per iteration from the host).
+// MPS_SOLVER_CG64: the reference CG in FP64.
 // MPS_SOLVER_MIXED: CG whose iterations run in FP32 (FP32 matrix, FP32 SpMV and axpy with
 // FP32 accumulation, dot products accumulated in FP64) with reliable updates (Sleijpen &
 // van der Vorst 1996): when the recursive residual has dropped by `delta` since the last
@@ -210,6 +210,18 @@ __device__ __forceinline__ void store_loop_width(const CgOperands& o, int c, int
     if ((threadIdx.x & 31) == 0 && o.loop_w) o.loop_w[c] = out ? 0 : o.chunk[c] / kSellRows;
 }
 
+// Entries of chunk c past row i's length L: {i, 0}, so that the loops add all entries of a
+// chunk's width without a look at the lengths (a finite vector's sums stay the same).
+__device__ __forceinline__ void pad_row(const CgOperands& o, int c, int i, int L, int64_t at, bool fp32) {
+    const int width = o.chunk[c] / kSellRows;
+    for (int k = L; k < width; k++) {
+        const int64_t e = at + static_cast<int64_t>(k) * kSellRows;
+        const_cast<int32_t*>(o.col)[e] = i;
+        const_cast<double*>(o.val)[e] = 0.0;
+        if (fp32) const_cast<uint2*>(o.cv32)[e] = make_uint2(static_cast<unsigned>(i), 0u);
+    }
+}
+
 // ------------------------------------------------------------- CG64 kernels
 // Ap = A x; r = b - Ap; p = r; rr = r.r (Computer.hpp:1382-1385).  With `gate` (the
 // fallback after a preconditioned solve) nothing runs unless that solve failed.
@@ -244,51 +256,12 @@ __global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, const CgScalar
             vbb += bi * bi;
         }
         store_loop_width(o, c, i, L, at, ri);
+        pad_row(o, c, i, L, at, false);
     }
     double tot[3];
     if (grid_sum(vrr, vbb, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) init_scalars(o.S, tot[0], tot[1], 0, 0);
 }
 
-// x += alpha p; r -= alpha Ap; rrNew = r.r; convergence; beta (Computer.hpp:1402-1420)
-__global__ void __launch_bounds__(kBlock) k_cg_update(CgOperands o) {
-    __shared__ BlockTicket tk;
-    if (cg_done(o.S)) return;
-    ticket_init(tk);
-    const double alpha = o.S->alpha;
-    double v = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x) {
-        o.x[i] = fma(alpha, o.p[i], o.x[i]);
-        const double ri = fma(-alpha, o.Ap[i], o.r[i]);
-        o.r[i] = ri;
-        v += ri * ri;
-    }
-    double tot[3];
-    if (grid_sum(v, 0.0, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) {
-        const double rr_new = tot[0];
-        {
-            CgScalars* S = o.S;
-            S->counter = 0;
-            S->rr_new = rr_new;
-            const int conv = rr_new < S->thr;
-            S->converged = conv;
-            if (!conv) {
-                S->beta = rr_new / S->rr;
-                S->rr = rr_new;
-            }
-            S->iter += 1;
-        }
-    }
-}
-
-// p = r + beta p
-__global__ void __launch_bounds__(kBlock) k_cg_pupdate(CgOperands o) {
-    if (cg_done(o.S)) return;
-    const double beta = o.S->beta;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x)
-        o.p[i] = fma(beta, o.p[i], o.r[i]);
-}
-
-// |b - A x|^2 in FP64 into S->true_rr (reported as the true relative residual)
 // |b - A x|^2 in FP64 for the statistics.  With `after_update` (the mixed-precision
 // solves) a solve that converged on its own already holds it: convergence is only ever
 // declared by a reliable update, on the true residual of the x it leaves.
@@ -326,9 +299,10 @@ __global__ void __launch_bounds__(kBlock) k_true_residual(CgOperands o, int afte
 // followed by the SpMV w = A r that also forms gamma and delta and the next step sizes.
 
 // init: r_0 = b - A x (FP64); r32 = r_0; d = 0; p = 0; s = 0; rr, bb
-// (plain: MIXED, whose loop leaves some rows out: both solution buffers hold their x)
+// (plain: MIXED, whose loop leaves some rows out: both solution buffers hold their x; pads:
+// a single-launch loop follows)
 __global__ void __launch_bounds__(kBlock) k_mx_init(CgOperands o, cudaGraphConditionalHandle h,
-                                                   int use_cond, int plain) {
+                                                   int use_cond, int plain, int pads) {
     __shared__ BlockTicket tk;
     if (aborted_before_solve(o, h, use_cond)) return;
     clear_slots(o.slots);
@@ -355,40 +329,18 @@ __global__ void __launch_bounds__(kBlock) k_mx_init(CgOperands o, cudaGraphCondi
             vbb += bi * bi;
         }
         if (plain) store_loop_width(o, c, i, L, at, ri);
+        if (pads) pad_row(o, c, i, L, at, true);
     }
     double tot[3];
     if (grid_sum(vrr, vbb, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) init_scalars(o.S, tot[0], tot[1], h, use_cond);
 }
 
-// s = w + beta s; p = r + beta p; d += alpha p; r -= alpha s (FP32, no reduction)
-__global__ void __launch_bounds__(kBlock) k_mx_axpy(CgOperands o) {
-    if (cg_done(o.S)) return;
-    const float alpha = __double2float_rn(o.S->alpha);
-    const float beta = __double2float_rn(o.S->beta);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < o.n; i += gridDim.x * blockDim.x) {
-        const float ri = o.r32[i];
-        const float si = fmaf(beta, o.s32[i], o.w32[i]);
-        const float pi = fmaf(beta, o.p32[i], ri);
-        o.s32[i] = si;
-        o.p32[i] = pi;
-        o.d32[i] = fmaf(alpha, pi, o.d32[i]);
-        o.r32[i] = fmaf(-alpha, si, ri);
-    }
-}
-
-// w = A r (FP32); gamma = r.r and delta = w.r in FP64; the next Chronopoulos-Gear step
-// sizes; decides a reliable update.  mode 0: after init (beta = 0); mode 1: an
-// iteration; mode 2: after a reliable update (also clears d, folded into x).
-__global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode) {
+// w = A r (FP32); gamma = r.r and delta = w.r in FP64; the first Chronopoulos-Gear step
+// size.  The iterations follow in k_mx_loop.
+__global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o) {
     __shared__ BlockTicket tk;
     CgScalars* S = o.S;
-    if (mode == 2) {
-        if (S->converged || S->aborted || !S->do_update) return;
-    } else if (mode == 1) {
-        if (cg_done(S)) return;
-    } else if (S->converged || S->aborted) {
-        return;
-    }
+    if (S->converged || S->aborted) return;
     ticket_init(tk);
     const ChunkLoop cl;
     const float* __restrict__ r = o.r32;
@@ -400,49 +352,18 @@ __global__ void __launch_bounds__(kBlock) k_mx_spmv(CgOperands o, int mode) {
         if (i < o.n) {
             const double ri = static_cast<double>(r[i]);
             o.w32[i] = wi;
-            if (mode == 2) o.d32[i] = 0.0f;
             vg += ri * ri;
             vd += static_cast<double>(wi) * ri;
         }
     }
     double tot[3];
     if (grid_sum(vg, vd, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) {
-        const double gam = tot[0];
-        const double del = tot[1];
-        {
-            S->counter = 0;
-            S->rr_new = gam;
-            int reliable = 0;
-            if (mode == 1) {
-                reliable = (gam < S->delta2 * S->rr_upd) || (gam < S->thr);
-                S->do_update = reliable;
-            }
-            if (!reliable) {
-                if (mode == 0) {
-                    S->beta = 0.0;
-                    S->alpha = gam / del;
-                } else {
-                    const double beta = gam / S->rr;
-                    S->beta = beta;
-                    S->alpha = gam / (del - beta * gam / S->alpha);
-                    S->iter += 1;
-                    // no tenfold drop of the recursive residual for kMixedStallIter
-                    // iterations: the FP32 iteration has stalled (the FP64 CG takes over)
-                    const int stuck = S->iter - S->iter_upd > kMixedStallIter;
-                    if (stuck) S->stalled = 1;
-                }
-                S->rr = gam;
-                S->pAp = del;
-            }
-            if (mode == 2) {
-                // after a reliable update: the true residual must at least halve in norm
-                // between updates, or the FP32 iteration has stalled (the FP64 CG takes over)
-                const int stalled = S->true_rr > 0.25 * S->prev_true_rr;
-                S->prev_true_rr = S->true_rr;
-                S->stalled = stalled;
-                S->do_update = 0;
-            }
-        }
+        S->counter = 0;
+        S->rr_new = tot[0];
+        S->beta = 0.0;
+        S->alpha = tot[0] / tot[1];
+        S->rr = tot[0];
+        S->pAp = tot[1];
     }
 }
 
@@ -1192,39 +1113,19 @@ __global__ void __launch_bounds__(kBlock, 4) k_pcg_persistent(CgOperands o, MgHi
 
 bool is_pcg(int solver) { return solver == MPS_SOLVER_MIXED_MG || solver == MPS_SOLVER_LEARNED; }
 
-void cg64_body(const CgOperands& ops, cudaStream_t s) {
-    launch_cg_spmv(ops, s);
-    k_cg_update<<<ops.grid_vec, kBlock, 0, s>>>(ops);
-    k_cg_pupdate<<<ops.grid_vec, kBlock, 0, s>>>(ops);
-}
-
-void reliable_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
-                      cudaGraphConditionalHandle h, int use_cond, cudaStream_t s) {
+void reliable_kernels(const CgOperands& ops, const MgHierarchy& mg, cudaGraphConditionalHandle h, int use_cond,
+                      cudaStream_t s) {
     launch_mx_true(ops, h, use_cond, s);
-    if (is_pcg(solver)) {
-        mg_apply(*mg, ops.S, 2, ops.r32, ops.u32, s);
-        launch_pmx_spmv(ops, 2, h, 0, use_cond, s, false);
-    } else {
-        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops, 2);
-    }
+    mg_apply(mg, ops.S, 2, ops.r32, ops.u32, s);
+    launch_pmx_spmv(ops, 2, h, 0, use_cond, s, false);
 }
 
-void body_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
-                  cudaGraphConditionalHandle h, cudaGraphConditionalHandle h_true, int use_cond,
-                  bool with_true, cudaStream_t s) {
-    const int gv = ops.grid_vec, gs = ops.grid_spmv;
-    if (solver == MPS_SOLVER_CG64) {
-        cg64_body(ops, s);
-        return;
-    }
-    if (is_pcg(solver)) {
-        mg_apply(*mg, ops.S, 1, ops.r32, ops.u32, s, &ops);  // vector updates + u = M r
-        launch_pmx_spmv(ops, 1, h, h_true, use_cond, s, true);
-    } else {
-        k_mx_axpy<<<gv, kBlock, 0, s>>>(ops);
-        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops, 1);
-    }
-    if (with_true) reliable_kernels(solver, ops, mg, h, use_cond, s);
+// An iteration of the preconditioned solvers.
+void body_kernels(const CgOperands& ops, const MgHierarchy& mg, cudaGraphConditionalHandle h,
+                  cudaGraphConditionalHandle h_true, int use_cond, bool with_true, cudaStream_t s) {
+    mg_apply(mg, ops.S, 1, ops.r32, ops.u32, s, &ops);  // vector updates + u = M r
+    launch_pmx_spmv(ops, 1, h, h_true, use_cond, s, true);
+    if (with_true) reliable_kernels(ops, mg, h, use_cond, s);
 }
 
 // The learned start in two parts: r0 of the previous pressure and the per-particle
@@ -1233,7 +1134,7 @@ void body_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
 void learned_prep_head(const LearnedOps& L, const CgOperands& o, CgScalars* S, cudaStream_t s) {
     CgOperands p = o;
     p.S = S;
-    k_mx_init<<<o.grid_spmv, kBlock, 0, s>>>(p, 0, 0, 0);  // r0 = b - A x0 in FP64, into r32
+    k_mx_init<<<o.grid_spmv, kBlock, 0, s>>>(p, 0, 0, 0, 0);  // r0 = b - A x0 in FP64, into r32
     launch_learned_q(L, p, S, s);
 }
 
@@ -1252,12 +1153,13 @@ void learned_prep_tail(const LearnedOps& L, const CgOperands& o, const MgHierarc
     }
 }
 
+// With `one_launch` the loop launch that follows makes the first preconditioned step itself.
 // With `fk` (graph capture), the coarse half of the multigrid setup runs on a side
 // stream beside the initial residual (and the learned start's first kernels), joining
 // before the first use of the hierarchy.  The two branches share no buffers.
 void init_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
                   cudaGraphConditionalHandle h, int use_cond, cudaStream_t s,
-                  const LearnedRun* lrn, const SetupFork* fk = nullptr) {
+                  const LearnedRun* lrn, const SetupFork* fk = nullptr, bool one_launch = false) {
     const int gs = ops.grid_spmv;
     if (solver == MPS_SOLVER_CG64) {
         k_cg_init<<<gs, kBlock, 0, s>>>(ops, nullptr);
@@ -1266,7 +1168,7 @@ void init_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
     const bool pcg = is_pcg(solver);
     const bool forked = pcg && fk != nullptr;
     if (pcg) {
-        mg_setup_level1(*mg, ops, s);
+        mg_setup_level1(*mg, ops, s, !one_launch || solver == MPS_SOLVER_LEARNED);
         if (forked) {
             cudaEventRecord(fk->fork, s);
             cudaStreamWaitEvent(fk->side, fk->fork, 0);
@@ -1281,16 +1183,17 @@ void init_kernels(int solver, const CgOperands& ops, const MgHierarchy* mg,
         learned_prep_head(*lrn->L, ops, lrn->S, s);
         if (forked) cudaStreamWaitEvent(s, fk->join, 0);
         learned_prep_tail(*lrn->L, ops, *mg, lrn->S, true, s);
-        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, pcg ? 0 : 1);
+        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, pcg ? 0 : 1, one_launch ? 1 : 0);
     } else {
-        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, pcg ? 0 : 1);
+        k_mx_init<<<gs, kBlock, 0, s>>>(ops, h, use_cond, pcg ? 0 : 1, one_launch ? 1 : 0);
         if (forked) cudaStreamWaitEvent(s, fk->join, 0);
     }
+    if (pcg && one_launch) return;
     if (pcg) {
         mg_apply(*mg, ops.S, 0, ops.r32, ops.u32, s);
         launch_pmx_spmv(ops, 0, h, 0, use_cond, s, false);
     } else {
-        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops, 0);
+        k_mx_spmv<<<gs, kBlock, 0, s>>>(ops);
     }
 }
 
@@ -1335,7 +1238,7 @@ void launch_spmv_only(int solver, const CgOperands& ops, cudaStream_t s) {
     else if (is_pcg(solver))
         launch_pmx_spmv(ops, 1, 0, 0, 0, s, false);
     else
-        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops, 1);
+        k_mx_spmv<<<ops.grid_spmv, kBlock, 0, s>>>(ops);
 }
 
 void learned_prep(const LearnedOps& L, const CgOperands& o, const MgHierarchy& mg, CgScalars* S,
@@ -1348,15 +1251,9 @@ int learned_prep_launches(const MgHierarchy& mg, bool infer) {
     return 1 + mg_apply_launches(mg) + 1 + 2 + (infer ? 2 : 0);
 }
 
-int cg_kernels_per_iteration(int solver, const MgHierarchy* mg) {
-    if (solver == MPS_SOLVER_CG64) return 3;
-    return is_pcg(solver) && mg ? 1 + mg_apply_launches(*mg) : 2;
-}
+int pcg_kernels_per_iteration(const MgHierarchy& mg) { return 1 + mg_apply_launches(mg); }
 
-int cg_kernels_per_update(int solver, const MgHierarchy* mg) {
-    if (solver == MPS_SOLVER_CG64) return 0;
-    return is_pcg(solver) && mg ? kMxTrueLaunches + 1 + mg_apply_launches(*mg) : kMxTrueLaunches + 1;
-}
+int pcg_kernels_per_update(const MgHierarchy& mg) { return kMxTrueLaunches + 1 + mg_apply_launches(mg); }
 
 CgGraph::~CgGraph() {
     reset();
@@ -1373,17 +1270,7 @@ void CgGraph::reset() {
     solver_ = -1;
     nested_ = false;
     persistent_ = false;
-}
-
-cudaError_t CgGraph::build(int solver, const CgOperands& ops, cudaStream_t s, const MgHierarchy* mg,
-                           const CgOperands* fb, const LearnedRun* lrn) {
-    if (!is_pcg(solver)) return build_plain(solver, ops, s, fb);
-    if (!mg || !fb) return cudaErrorInvalidValue;
-    if (solver == MPS_SOLVER_LEARNED && !lrn) return cudaErrorInvalidValue;
-    // preferred: the reliable update under an IF node nested in the WHILE body
-    if (build_impl(solver, ops, s, true, mg, fb, lrn) == cudaSuccess) return cudaSuccess;
-    cudaGetLastError();
-    return build_impl(solver, ops, s, false, mg, fb, lrn);
+    one_launch_ = false;
 }
 
 namespace {
@@ -1398,36 +1285,84 @@ cudaError_t fallback_kernels(const CgOperands& ops, const CgOperands& fb, int af
 }
 }  // namespace
 
-// CG64 and MIXED: init, the loop in one launch (cgloop.cu), [the FP64 CG after a failed
+namespace {
+// Whether the solver's iteration loop is one launch: where its block's share fits shared
+// memory it was faster at every size measured (pcgloop.cu).
+bool loops_in_one_launch(int solver, const MgHierarchy* mg) {
+    return !is_pcg(solver) || pcg_loop_fits(*mg);
+}
+
+// Init kernels, the loop in one launch (cgloop.cu, pcgloop.cu), [the FP64 CG after a failed
 // mixed loop], the true residual.
-cudaError_t CgGraph::build_plain(int solver, const CgOperands& ops, cudaStream_t s, const CgOperands* fb) {
-    reset();
-    ops_ = ops;
-    solver_ = solver;
-    cudaError_t e = cudaGraphCreate(&graph_, 0);
-    if (e != cudaSuccess) return e;
-    cudaGraph_t captured = nullptr;
-    e = cudaStreamBeginCaptureToGraph(s, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
-    init_kernels(solver, ops, nullptr, 0, 0, s, nullptr);
-    cudaError_t le;
+cudaError_t one_launch_kernels(int solver, const CgOperands& ops, cudaStream_t s, const MgHierarchy* mg,
+                               const CgOperands* fb, const LearnedRun* lrn, const SetupFork* fk) {
+    init_kernels(solver, ops, mg, 0, 0, s, lrn, fk, true);
+    cudaError_t e;
     if (solver == MPS_SOLVER_CG64) {
-        le = launch_cg_loop(ops, s);
-    } else {
-        le = launch_mx_loop(ops, s);
+        e = launch_cg_loop(ops, s);
+    } else if (solver == MPS_SOLVER_MIXED) {
+        e = launch_mx_loop(ops, s);
         k_mx_finish<<<ops.grid_vec, kBlock, 0, s>>>(ops);
+    } else {
+        e = launch_pcg_loop(ops, *mg, s);
     }
     if (solver != MPS_SOLVER_CG64 && fb) {
-        const cudaError_t fe = fallback_kernels(ops, *fb, 1, s);
-        if (le == cudaSuccess) le = fe;
+        const cudaError_t f = fallback_kernels(ops, *fb, 1, s);
+        if (e == cudaSuccess) e = f;
     } else {
         k_true_residual<<<ops.grid_spmv, kBlock, 0, s>>>(ops, solver != MPS_SOLVER_CG64 ? 1 : 0);
     }
+    return e;
+}
+}  // namespace
+
+int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb) {
+    const int tail = with_fb ? 4 : 1;  // the fallback's init, loop and merge; the true residual
+    if (solver == MPS_SOLVER_CG64) return 2 + 1;
+    if (solver == MPS_SOLVER_MIXED) return 4 + tail;
+    const bool learned = solver == MPS_SOLVER_LEARNED;
+    return mg_setup_launches(*mg, learned) + 2 + tail + (learned ? 1 + learned_prep_launches(*mg, true) : 0);
+}
+
+cudaError_t CgGraph::build(int solver, const CgOperands& ops, cudaStream_t s, const MgHierarchy* mg,
+                           const CgOperands* fb, const LearnedRun* lrn) {
+    if (is_pcg(solver) && (!mg || !fb)) return cudaErrorInvalidValue;
+    if (solver == MPS_SOLVER_LEARNED && !lrn) return cudaErrorInvalidValue;
+    if (loops_in_one_launch(solver, mg)) return build_one_launch(solver, ops, s, mg, fb, lrn);
+    // preferred: the reliable update under an IF node nested in the WHILE body
+    if (build_impl(solver, ops, s, true, mg, fb, lrn) == cudaSuccess) return cudaSuccess;
+    cudaGetLastError();
+    return build_impl(solver, ops, s, false, mg, fb, lrn);
+}
+
+cudaError_t CgGraph::build_one_launch(int solver, const CgOperands& ops, cudaStream_t s, const MgHierarchy* mg,
+                                      const CgOperands* fb, const LearnedRun* lrn) {
+    reset();
+    ops_ = ops;
+    solver_ = solver;
+    one_launch_ = true;
+    cudaError_t e = cudaGraphCreate(&graph_, 0);
+    if (e != cudaSuccess) return e;
+    cudaGraph_t captured = nullptr;
+    e = make_fork();
+    if (e != cudaSuccess) return e;
+    e = cudaStreamBeginCaptureToGraph(s, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    const cudaError_t le = one_launch_kernels(solver, ops, s, mg, fb, lrn, &fork_);
     e = cudaStreamEndCapture(s, &captured);
     if (le != cudaSuccess) return le;
     if (e != cudaSuccess) return e;
     e = cudaGraphInstantiate(&exec_, graph_, 0);
     if (e != cudaSuccess) exec_ = nullptr;
+    return e;
+}
+
+// Side stream and events of the multigrid setup's branch.
+cudaError_t CgGraph::make_fork() {
+    if (fork_.side) return cudaSuccess;
+    cudaError_t e = cudaStreamCreateWithFlags(&fork_.side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork_.fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork_.join, cudaEventDisableTiming);
     return e;
 }
 
@@ -1482,8 +1417,8 @@ cudaError_t CgGraph::build_impl(int solver, const CgOperands& ops, cudaStream_t 
     ops_ = ops;
     solver_ = solver;
     nested_ = nested;
-    kpi_ = cg_kernels_per_iteration(solver, mg);
-    kri_ = cg_kernels_per_update(solver, mg);
+    kpi_ = pcg_kernels_per_iteration(*mg);
+    kri_ = pcg_kernels_per_update(*mg);
     cudaError_t e = cudaGraphCreate(&graph_, 0);
     if (e != cudaSuccess) return e;
     cudaGraphConditionalHandle h;
@@ -1492,12 +1427,8 @@ cudaError_t CgGraph::build_impl(int solver, const CgOperands& ops, cudaStream_t 
     cudaGraph_t captured = nullptr;
 
     // init chain (the multigrid's coarse setup on a side branch)
-    if (!fork_.side) {
-        e = cudaStreamCreateWithFlags(&fork_.side, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork_.fork, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork_.join, cudaEventDisableTiming);
-        if (e != cudaSuccess) return e;
-    }
+    e = make_fork();
+    if (e != cudaSuccess) return e;
     e = cudaStreamBeginCaptureToGraph(s, graph_, nullptr, nullptr, 0,
                                       cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
@@ -1520,7 +1451,7 @@ cudaError_t CgGraph::build_impl(int solver, const CgOperands& ops, cudaStream_t 
     }
     e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    body_kernels(solver, ops, mg, h, h_true, 1, !nested, s);
+    body_kernels(ops, *mg, h, h_true, 1, !nested, s);
     e = cudaStreamEndCapture(s, &captured);
     if (e != cudaSuccess) return e;
 
@@ -1541,7 +1472,7 @@ cudaError_t CgGraph::build_impl(int solver, const CgOperands& ops, cudaStream_t 
         e = cudaStreamBeginCaptureToGraph(s, if_body, nullptr, nullptr, 0,
                                           cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
-        reliable_kernels(solver, ops, mg, h, 1, s);
+        reliable_kernels(ops, *mg, h, 1, s);
         e = cudaStreamEndCapture(s, &captured);
         if (e != cudaSuccess) return e;
     }
@@ -1628,59 +1559,38 @@ cudaError_t CgGraph::launch(cudaStream_t s) {
     return cudaGraphLaunch(exec_, s);
 }
 
-namespace {
-// Host loop: `chunk` iterations per batch, the scalars read back between batches.
-cudaError_t host_loop(int solver, const CgOperands& ops, const MgHierarchy* mg, CgScalars* host_S,
-                      int chunk, cudaStream_t s, int64_t* k) {
-    const cudaGraphConditionalHandle none = 0;
-    cudaError_t e = cudaGetLastError();
-    for (;;) {
-        if (e != cudaSuccess) return e;
-        e = cudaMemcpyAsync(host_S, ops.S, sizeof(CgScalars), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return e;
-        if (host_S->converged || host_S->aborted || host_S->stalled || host_S->iter >= host_S->max_iter)
-            return cudaSuccess;
-        for (int c = 0; c < chunk; c++) {
-            body_kernels(solver, ops, mg, none, none, 0, true, s);
-            // every kernel of the iteration and of the reliable update is launched
-            *k += cg_kernels_per_iteration(solver, mg) + cg_kernels_per_update(solver, mg);
-        }
-        e = cudaGetLastError();
-    }
-}
-}  // namespace
-
 cudaError_t cg_run_direct(int solver, const CgOperands& ops, CgScalars* host_S, int chunk,
                           cudaStream_t s, int64_t* launches, const MgHierarchy* mg,
                           const CgOperands* fb, const LearnedRun* lrn) {
     if (is_pcg(solver) && (!mg || !fb)) return cudaErrorInvalidValue;
     if (solver == MPS_SOLVER_LEARNED && !lrn) return cudaErrorInvalidValue;
-    const int gv = ops.grid_vec, gs = ops.grid_spmv;
+    if (loops_in_one_launch(solver, mg)) {
+        const cudaError_t e = one_launch_kernels(solver, ops, s, mg, fb, lrn, nullptr);
+        if (launches) *launches = one_launch_count(solver, mg, fb != nullptr);
+        return e == cudaSuccess ? cudaGetLastError() : e;
+    }
     const cudaGraphConditionalHandle none = 0;
-    int64_t k = 0;
+    int64_t k = 2 + mg_setup_launches(*mg) + mg_apply_launches(*mg);
     init_kernels(solver, ops, mg, none, 0, s, lrn);
-    k += solver == MPS_SOLVER_CG64 ? 1 : 2;
-    if (is_pcg(solver)) k += mg_setup_launches(*mg) + mg_apply_launches(*mg);
     if (solver == MPS_SOLVER_LEARNED) k += 1 + learned_prep_launches(*mg, true);
-    cudaError_t e = host_loop(solver, ops, mg, host_S, chunk, s, &k);
-    if (e != cudaSuccess) return e;
-    if (solver != MPS_SOLVER_CG64) {
-        k_mx_finish<<<gv, kBlock, 0, s>>>(ops);
-        k++;
-    }
-    if (solver != MPS_SOLVER_CG64 && fb) {
-        k_cg_init<<<gs, kBlock, 0, s>>>(*fb, ops.S);
-        k++;
-        e = host_loop(MPS_SOLVER_CG64, *fb, nullptr, host_S, chunk, s, &k);
+    cudaError_t e = cudaGetLastError();
+    for (;;) {  // `chunk` iterations per batch, the scalars read back between batches
         if (e != cudaSuccess) return e;
-        k_fb_merge<<<1, 32, 0, s>>>(ops.S, fb->S);
-        k++;
+        e = cudaMemcpyAsync(host_S, ops.S, sizeof(CgScalars), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
+        if (host_S->converged || host_S->aborted || host_S->stalled || host_S->iter >= host_S->max_iter) break;
+        for (int c = 0; c < chunk; c++) {
+            body_kernels(ops, *mg, none, none, 0, true, s);
+            // every kernel of the iteration and of the reliable update is launched
+            k += pcg_kernels_per_iteration(*mg) + pcg_kernels_per_update(*mg);
+        }
+        e = cudaGetLastError();
     }
-    k_true_residual<<<gs, kBlock, 0, s>>>(ops, solver != MPS_SOLVER_CG64 ? 1 : 0);
-    k++;
-    if (launches) *launches = k;
-    return cudaGetLastError();
+    k_mx_finish<<<ops.grid_vec, kBlock, 0, s>>>(ops);
+    e = fallback_kernels(ops, *fb, 1, s);
+    if (launches) *launches = k + 5;
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace mpsgb

@@ -256,6 +256,7 @@ public:
     cudaError_t launch(cudaStream_t s);
     void reset();
     bool persistent() const { return persistent_; }
+    bool one_launch() const { return one_launch_; }  // the iteration loop is one launch
     bool valid() const { return exec_ != nullptr; }
     int solver() const { return solver_; }
     const CgOperands& operands() const { return ops_; }
@@ -265,30 +266,32 @@ public:
     bool nested() const { return nested_; }
 
 private:
-    cudaError_t build_plain(int solver, const CgOperands& ops, cudaStream_t s, const CgOperands* fb);
+    cudaError_t build_one_launch(int solver, const CgOperands& ops, cudaStream_t s, const MgHierarchy* mg,
+                                 const CgOperands* fb, const LearnedRun* lrn);
     cudaError_t build_impl(int solver, const CgOperands& ops, cudaStream_t s, bool nested,
                            const MgHierarchy* mg, const CgOperands* fb, const LearnedRun* lrn);
+    cudaError_t make_fork();
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     int solver_ = -1;
     bool nested_ = false;
     bool persistent_ = false;
+    bool one_launch_ = false;
     int kpi_ = 0, kri_ = 0;
     CgOperands ops_{};
     SetupFork fork_;  // created at the first build, kept across rebuilds
 };
 
-// The same solve with host-launched kernels: `chunk` iterations per launch batch, the
+// The same solve with host-launched kernels, which profilers see one by one (the same
+// results).  A loop that is not one launch runs `chunk` iterations per launch batch, with the
 // device status read back between batches (kernels past convergence return at once).
-// Used when kernels must be visible one by one (profilers) and as a fallback.
 cudaError_t cg_run_direct(int solver, const CgOperands& ops, CgScalars* host_S, int chunk,
                           cudaStream_t s, int64_t* launches, const MgHierarchy* mg = nullptr,
                           const CgOperands* fb = nullptr, const LearnedRun* lrn = nullptr);
 // Grid size of the persistent solve on the current device (0: cooperative launch unavailable).
 int persistent_blocks();
-// Kernels of one iteration of the solver, and of one reliable update.
-int cg_kernels_per_iteration(int solver, const MgHierarchy* mg);
-int cg_kernels_per_update(int solver, const MgHierarchy* mg);
+// Kernels of a solve whose loop is one launch (with_fb: and the fallback's).
+int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb);
 
 // Sets eps / criterion / max_iter / delta for the next solve (stream-ordered).
 void launch_cg_configure(CgScalars* S, double eps, int criterion, int max_iter, double delta2,

@@ -6,32 +6,24 @@
 // rows are even over the blocks; chunks of identity rows with a zero residual (dummy and
 // disabled particles: 84 % of the 3D dam break's chunks) keep x and stay out of the loop.
 // The split stays the same through the solve, so a row's vectors are touched by one thread
-// only, and the block keeps them in shared memory when they fit (the gathered vector has
-// its global copy).  For a product A v the block's chunks are cut into units of a few
-// entries of a chunk's 32 rows (one warp per unit, one lane per row), the unit sums are
-// parked in shared memory and the row's thread adds them: with whole chunks per warp, 17
-// chunks of 46 entries (84k rows over 152 SMs) would occupy 17 of 32 warps, and a 58-chunk
-// system (1,850 rows) would wait for one lane's 46 dependent multiply-adds.  Blocks with
-// more chunks than the sums' room take them in tiles.
+// only, and the block keeps them in shared memory when they fit (the gathered vector has its
+// global copy).
 //
 // CG64: the reference's conjugate gradient (Computer.hpp:1359-1429) with two grid-wide
 // exchanges per iteration instead of three: the product is formed with the residual, and
 // A p follows from s = A r + beta s (p = r + beta p), so p needs no exchange of its own.
 // Both dot products are formed from the vectors themselves, as in the reference.
-// MIXED: the Chronopoulos-Gear iteration of cg.cu (k_mx_axpy, k_mx_spmv, the reliable
-// update of k_mx_fold and the FP64 true residual), phase by phase.
-
-#include "cg.cuh"
-#include "gridloop.cuh"
+// MIXED: Chronopoulos-Gear CG in FP32 with FP64 dot products and reliable updates (cg.cu).
+#include "cgloop.cuh"
 
 namespace mpsgb {
 
 namespace {
 
-constexpr int kStep = 8;         // matrix entries a lane loads at once
-constexpr int kMaxUnits = 8;     // units of one chunk (longer rows take longer units)
-constexpr int kTileChunks = 40;  // chunks whose unit sums fit a tile (40 x 8 x 32 doubles = 80 KB)
+constexpr int kPartUnits = 320;  // unit sums of a tile (80 KB of doubles)
+constexpr int kTileChunks = kPartUnits / kMaxUnits;
 
+// dynamic shared memory: unit sums, chunk table, unit table, vectors
 struct LoopPlan {
     int blocks;
     int tables;      // chunks the tables hold: all that a block can own, or one tile
@@ -39,69 +31,8 @@ struct LoopPlan {
     size_t smem;
 };
 
-struct ChunkInfo {
-    int chunk, off, width, first;  // first: its first unit
-    int units, pad;
-};
-
-// dynamic shared memory: unit sums, chunk table, unit table, vectors
-struct LoopView {
-    double* part;     // kTileChunks * kMaxUnits * 32
-    ChunkInfo* info;  // all chunks of the block (whole) or those of a tile
-    int2* unit;       // {table index, first entry}
-    unsigned char* keep;
-    int c0, nc;  // whole: table entries are the chunks; else chunks c0 .. c0 + nc - 1
-    int tile;    // chunks per tile
-    int active;  // threads that own rows
-    int warps;
-    int cuts;  // units of a chunk, at most kMaxUnits
-    bool whole;
-};
-
 size_t table_bytes(int tables) {
-    return sizeof(double) * kTileChunks * kMaxUnits * 32 +
-           (sizeof(ChunkInfo) + sizeof(int2) * kMaxUnits) * static_cast<size_t>(tables);
-}
-
-// Entries of a unit of a chunk `width` entries wide.  A block with chunks to spare takes
-// them in few units (each unit past the first costs the row an addition); one with few
-// cuts them so that its warps all have one.
-__device__ __forceinline__ int unit_span(const LoopView& L, int width) {
-    const int per = (width + L.cuts - 1) / L.cuts;
-    return (per + kStep - 1) / kStep * kStep;
-}
-
-// Completes the table entries [0, m) whose chunks are set, and lists their units.
-__device__ __forceinline__ void build_tables(const CgOperands& o, const LoopView& L, int m) {
-    const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
-    for (int k = t; k < m; k += nt) {
-        const int c = L.info[k].chunk;
-        const int w = o.chunk[c] / kSellRows;
-        L.info[k].off = o.off[c];
-        L.info[k].width = w;
-        L.info[k].units = w > 0 ? (w + unit_span(L, w) - 1) / unit_span(L, w) : 0;
-    }
-    __syncthreads();
-    if (t < 32) {  // exclusive prefix sum of the unit counts
-        int run = 0;
-        for (int b = 0; b < m; b += 32) {
-            const int u = b + t < m ? L.info[b + t].units : 0;
-            int s = u;
-            for (int d = 1; d < 32; d <<= 1) {
-                const int x = __shfl_up_sync(0xffffffffu, s, d);
-                if (t >= d) s += x;
-            }
-            if (b + t < m) L.info[b + t].first = run + s - u;
-            run += __shfl_sync(0xffffffffu, s, 31);
-        }
-    }
-    __syncthreads();
-    for (int k = t; k < m; k += nt) {
-        const ChunkInfo c = L.info[k];
-        const int span = unit_span(L, c.width);
-        for (int u = 0; u < c.units; u++) L.unit[c.first + u] = make_int2(k, u * span);
-    }
-    __syncthreads();
+    return sizeof(double) * kPartUnits * 32 + static_cast<size_t>(kChunkBytes) * tables;
 }
 
 // This block's chunks.  o.loop_w[c] is the width of a chunk the loop works on, 0 for one it
@@ -109,13 +40,14 @@ __device__ __forceinline__ void build_tables(const CgOperands& o, const LoopView
 // floor(P_k G / P_N), P_k = (widths before it) + a (chunks before it), a = W / (4 N) (a
 // row's vector work is about ten matrix entries' at the 46 entries of the usual radius): a
 // block then owns at most 5 N / G + 1 chunks, and even shares when the widths are alike.
-__device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPlan& plan, unsigned char* sm) {
+__device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPlan& plan, unsigned char* sm,
+                                             unsigned char** keep) {
     __shared__ int wsum[32], wcnt[32], first_pos, last_pos, first_chunk, last_chunk;
     LoopView L;
+    L.lo = 0;
+    L.hi = o.n;
     L.part = reinterpret_cast<double*>(sm);
-    L.info = reinterpret_cast<ChunkInfo*>(L.part + kTileChunks * kMaxUnits * 32);
-    L.unit = reinterpret_cast<int2*>(L.info + plan.tables);
-    L.keep = reinterpret_cast<unsigned char*>(L.unit + static_cast<size_t>(plan.tables) * kMaxUnits);
+    *keep = place_tables(L, L.part + kPartUnits * 32, plan.tables);
     const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x), lane = t & 31;
     L.warps = nt >> 5;
     const int seg = (o.nchunks + nt - 1) / nt;
@@ -181,179 +113,9 @@ __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPla
             L.nc = L.whole ? mine : last_chunk - first_chunk + 1;
         }
     }
-    const int tiles = max(1, (L.nc + kTileChunks - 1) / kTileChunks);
-    L.tile = max(1, (L.nc + tiles - 1) / tiles);
-    L.active = min(nt, L.nc * 32);
-    L.cuts = min(kMaxUnits, max(1, (2 * L.warps + L.tile - 1) / L.tile));
+    split_tiles(L, kPartUnits, plan.tables);
     if (L.whole) build_tables(o, L, L.nc);
     return L;
-}
-
-// the SELL chunk of the block's k-th chunk
-__device__ __forceinline__ int chunk_of(const LoopView& L, int k) { return L.whole ? L.info[k].chunk : L.c0 + k; }
-
-__device__ __forceinline__ int ld_once(const int32_t* p) {
-    int v;
-    asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ double ld_once(const double* p) {
-    double v;
-    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-    return v;
-}
-
-// A step of a unit: up to kStep entries of the lane's row.
-template <class T>
-struct UnitStep {
-    int c[kStep];
-    T a[kStep];
-    int len;  // entries of the lane's row from the step on
-    int out;  // the unit, when this is its last step (else -1)
-};
-
-// The warp's steps in order.
-template <class T>
-struct UnitCursor {
-    const CgOperands& o;
-    const LoopView& L;
-    int u, u1, k0, end;
-    ChunkInfo ci;
-
-    __device__ __forceinline__ void open() {
-        const int2 un = L.unit[u];
-        ci = L.info[un.x];
-        k0 = un.y;
-        end = min(ci.width, k0 + unit_span(L, ci.width));
-    }
-    __device__ __forceinline__ UnitCursor(const CgOperands& o_, const LoopView& L_, int u_, int u1_)
-        : o(o_), L(L_), u(u_), u1(u1_), k0(0), end(0) {
-        if (u < u1) open();
-    }
-    __device__ __forceinline__ bool valid() const { return u < u1; }
-    // Loads the current step and moves on.  Entries of a row past its length lie inside
-    // the chunk: they are loaded, not used.
-    __device__ __forceinline__ void load(UnitStep<T>& s) {
-        const int lane = threadIdx.x & 31;
-        s.len = o.len[ci.chunk * kSellRows + lane] - k0;
-        const int64_t at = static_cast<int64_t>(ci.off) + static_cast<int64_t>(k0) * kSellRows + lane;
-#pragma unroll
-        for (int e = 0; e < kStep; e++) {
-            s.c[e] = 0;
-            s.a[e] = 0;
-            if (k0 + e < ci.width) {
-                if constexpr (sizeof(T) == 8) {
-                    s.c[e] = ld_once(o.col + at + e * kSellRows);
-                    s.a[e] = ld_once(o.val + at + e * kSellRows);
-                } else {
-                    const uint2 p = ld_sell_pair(o.cv32 + at + e * kSellRows);
-                    s.c[e] = static_cast<int>(p.x);
-                    s.a[e] = __uint_as_float(p.y);
-                }
-            }
-        }
-        s.out = -1;
-        k0 += kStep;
-        if (k0 >= end) {
-            s.out = u;
-            u += L.warps;
-            if (u < u1) open();
-        }
-    }
-};
-
-// Unit sums of table chunks [a, b): T = double (FP64 matrix) or float (FP32 pairs).  Two
-// steps in turn, each loaded while the other gathers and adds: a warp waits for one round
-// trip to L2 per step (0.6 us across the dies), not for two.
-template <class T>
-__device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L, int a, int b, const T* v) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* part = reinterpret_cast<T*>(L.part);
-    const int u0 = L.info[a].first, u1 = L.info[b - 1].first + L.info[b - 1].units;
-    UnitCursor<T> cur(o, L, u0 + warp, u1);
-    if (!cur.valid()) return;
-    T acc = 0;
-    auto add = [&](const UnitStep<T>& s) {
-        T xv[kStep];
-#pragma unroll
-        for (int e = 0; e < kStep; e++) xv[e] = e < s.len ? v[s.c[e]] : T(0);
-#pragma unroll
-        for (int e = 0; e < kStep; e++)
-            if (e < s.len) {
-                if constexpr (sizeof(T) == 8) acc = fma(s.a[e], xv[e], acc);
-                else acc = fmaf(s.a[e], xv[e], acc);
-            }
-        if (s.out >= 0) {
-            part[(s.out - u0) * 32 + lane] = acc;
-            acc = 0;
-        }
-    };
-    UnitStep<T> A, B;
-    cur.load(A);
-    while (true) {
-        const bool b_next = cur.valid();
-        if (b_next) cur.load(B);
-        add(A);
-        if (!b_next) break;
-        const bool a_next = cur.valid();
-        if (a_next) cur.load(A);
-        add(B);
-        if (!a_next) break;
-    }
-}
-
-// f(local row, row, (A v)_row) for every row of the block, by the row's thread
-template <class T, class F>
-__device__ __forceinline__ void product(const CgOperands& o, const LoopView& L, const T* v, F f) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const T* part = reinterpret_cast<const T*>(L.part);
-    for (int k0 = 0; k0 < L.nc; k0 += L.tile) {
-        const int k1 = min(L.nc, k0 + L.tile);
-        const int table0 = L.whole ? 0 : k0;
-        if (!L.whole) {
-            for (int k = k0 + static_cast<int>(threadIdx.x); k < k1; k += static_cast<int>(blockDim.x))
-                L.info[k - k0].chunk = L.c0 + k;
-            __syncthreads();
-            build_tables(o, L, k1 - k0);
-        }
-        unit_sums<T>(o, L, k0 - table0, k1 - table0, v);
-        __syncthreads();
-        const int u0 = L.info[k0 - table0].first;
-        const int skip = k0 % L.warps;  // chunk k belongs to warp k % warps
-        for (int k = k0 - skip + warp + (warp < skip ? L.warps : 0); k < k1; k += L.warps) {
-            const ChunkInfo c = L.info[k - table0];
-            const T* p = part + (c.first - u0) * 32 + lane;
-            T s = c.units > 0 ? p[0] : T(0);  // two chains of additions
-            if (c.units > 1) {
-                T q = p[32];
-                for (int u = 2; u < c.units; u++) {
-                    if (u & 1) q += p[u * 32];
-                    else s += p[u * 32];
-                }
-                s += q;
-            }
-            const int row = c.chunk * kSellRows + lane;
-            if (row < o.n) f(k * kSellRows + lane, row, s);
-        }
-        if (k1 < L.nc) __syncthreads();  // the next tile overwrites the sums
-    }
-}
-
-// g(local row, row) for every row of the block, by the thread product() gives it to
-template <class G>
-__device__ __forceinline__ void own_rows(const CgOperands& o, const LoopView& L, G g) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = warp; k < L.nc; k += L.warps) {
-        const int row = chunk_of(L, k) * kSellRows + lane;
-        if (row < o.n) g(k * kSellRows + lane, row);
-    }
-}
-
-__device__ __forceinline__ void loop_timeout(const CgOperands& o) {
-    if (threadIdx.x == 0) {
-        if (o.status) atomicOr(&const_cast<DevStatus*>(o.status)->flags, kStatusWaitTimeout);
-        o.S->aborted = 1;
-    }
 }
 
 template <bool kCluster>
@@ -366,7 +128,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
     } sc;
     CgScalars* S = o.S;
     if (S->converged || S->aborted || S->iter >= S->max_iter) return;
-    const LoopView L = loop_view(o, plan, loop_sm);
+    unsigned char* keep_sm;
+    const LoopView L = loop_view(o, plan, loop_sm, &keep_sm);
     if (kCluster) loop_cluster_start();
     LoopSync ls{o.slots, gridDim.x, 0};
     const double thr = S->thr;
@@ -381,7 +144,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
     // they are kept in shared memory, the row itself in the global arrays
     const int rows = L.nc * kSellRows;
     const bool keep = L.whole && 4 * static_cast<int64_t>(sizeof(double)) * rows <= plan.keep_bytes;
-    double* kept = reinterpret_cast<double*>(L.keep);
+    double* kept = reinterpret_cast<double*>(keep_sm);
     double* P = keep ? kept : o.p;
     double* Q = keep ? kept + rows : o.Ap;
     double* X = keep ? kept + 2 * rows : o.x;
@@ -402,7 +165,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
         double v = 0.0;
         {
             const double beta = sc.beta;
-            product<double>(o, L, o.r, [&](int local, int row, double ar) {
+            product<double>(o, L, [&](int j) { return o.r[j]; }, [&](int local, int row, double ar) {
                 const int a = keep ? local : row;
                 const double p = fma(beta, P[a], R[a]);
                 const double s = fma(beta, Q[a], ar);
@@ -466,15 +229,21 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     extern __shared__ __align__(16) unsigned char loop_sm[];
     __shared__ LoopReduce red;
     __shared__ CgScalars sc;  // the solve's scalars, as the per-phase kernels keep them
+    __shared__ float alpha32, beta32;
     if (o.S->converged || o.S->aborted || o.S->iter >= o.S->max_iter) return;
-    const LoopView L = loop_view(o, plan, loop_sm);
+    unsigned char* keep_sm;
+    const LoopView L = loop_view(o, plan, loop_sm, &keep_sm);
     if (kCluster) loop_cluster_start();
     LoopSync ls{o.slots, gridDim.x, 0};
-    if (threadIdx.x == 0) sc = *o.S;
+    if (threadIdx.x == 0) {
+        sc = *o.S;
+        alpha32 = __double2float_rn(sc.alpha);
+        beta32 = __double2float_rn(sc.beta);
+    }
     // the block's rows of s, p, d, w and r (kept or global, as in k_cg_loop)
     const int rows = L.nc * kSellRows;
     const bool keep = L.whole && 5 * static_cast<int64_t>(sizeof(float)) * rows <= plan.keep_bytes;
-    float* kept = reinterpret_cast<float*>(L.keep);
+    float* kept = reinterpret_cast<float*>(keep_sm);
     float* Sv = keep ? kept : o.s32;
     float* Pv = keep ? kept + rows : o.p32;
     float* Dv = keep ? kept + 2 * rows : o.d32;
@@ -492,13 +261,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     // w = A r (FP32); gamma = r.r and delta = w.r in FP64, and what follows from them
     auto spmv = [&](bool after_update) {
         double v[2] = {0.0, 0.0};
-        product<float>(o, L, o.r32, [&](int local, int row, float w) {
+        product<float>(o, L, [&](int j) { return o.r32[j]; }, [&](int local, int row, float w) {
             const int a = keep ? local : row;
-            const double ri = static_cast<double>(Rv[a]);
+            const double ri = widen(Rv[a]);
             Wv[a] = w;
             if (after_update) Dv[a] = 0.0f;
             v[0] = fma(ri, ri, v[0]);
-            v[1] = fma(static_cast<double>(w), ri, v[1]);
+            v[1] = fma(widen(w), ri, v[1]);
         });
         return loop_reduce<kCluster, 2>(ls, red, v, L.active, [&](const double* tot) {
             const double gam = tot[0], del = tot[1];
@@ -513,6 +282,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
             if (!sc.do_update) {
                 sc.beta = q;
                 sc.alpha = alpha;
+                alpha32 = __double2float_rn(alpha);  // once: a conversion takes the pipe 64 cycles a warp
+                beta32 = __double2float_rn(q);
                 sc.iter += 1;
                 if (sc.iter - sc.iter_upd > kMixedStallIter) sc.stalled = 1;
                 sc.rr = gam;
@@ -529,7 +300,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     while (ok && !sc.stalled && sc.iter < sc.max_iter) {
         {
             // s = w + beta s; p = r + beta p; d += alpha p; r -= alpha s
-            const float alpha = __double2float_rn(sc.alpha), beta = __double2float_rn(sc.beta);
+            const float alpha = alpha32, beta = beta32;
             own_rows(o, L, [&](int local, int row) {
                 const int a = keep ? local : row;
                 const float si = fmaf(beta, Sv[a], Wv[a]);
@@ -554,7 +325,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
         ok = loop_reduce<kCluster, 0>(ls, red, nullptr, 0, [](const double*) {});
         if (!ok) break;
         double v = 0.0;
-        product<double>(o, L, xn, [&](int local, int row, double ax) {
+        product<double>(o, L, [&](int j) { return xn[j]; }, [&](int local, int row, double ax) {
             const double ri = o.b[row] - ax;
             const float rf = __double2float_rn(ri);
             Rv[keep ? local : row] = rf;
@@ -588,10 +359,10 @@ size_t g_loop_smem = 0;    // largest dynamic shared memory of a block
 // SMs have a tenth of the FP64 pipes and of the loads in flight.  us per iteration, cluster
 // against grid (dam breaks at r_e = 4 l0; the WHILE node's kernels took 29-31 and 19-21):
 //   rows      1,850        3,133        5,250         9,403
-//   CG64    6.8 / 8.2    8.7 / 8.3   11.2 / 8.5    16.8 / 8.9
-//   MIXED   5.5 / 7.1    6.7 / 7.3    8.2 / 7.2    11.1 / 7.2
-// The grid form at 16,850, 42,226, 90,050 and 340,050 rows: CG64 10.2, 14.9, 23.0, 72.9
-// (WHILE: 30.4, 31.5, 37.2, 73.7), MIXED 7.7, 10.7, 16.4 (20.6, 21.7, 25.1); the FP64 pipe
+//   CG64    6.4 / 8.2    8.7 / 8.0   11.2 / 8.1    16.8 / 8.6
+//   MIXED   5.5 / 7.1    6.1 / 7.3    8.2 / 7.1    11.1 / 7.1
+// The grid form at 16,850, 42,226, 90,050 and 340,050 rows: CG64 9.7, 13.5, 21.9, 58.0
+// (WHILE: 30.4, 31.5, 37.2, 73.7), MIXED 8.0, 9.4, 16.4 (20.6, 21.7, 25.1); the FP64 pipe
 // bounds the large CG64 systems (one multiply-add per entry: 6.4 us at 90,050 rows), the
 // exchanges the small ones.
 constexpr int kClusterChunks64 = 80, kClusterChunks32 = 128;

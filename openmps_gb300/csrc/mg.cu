@@ -107,9 +107,12 @@ __device__ __forceinline__ void store_level(const MgLevel& L, int c, const doubl
     L.dinv[c] = k[4] < 0.0 ? omega / static_cast<float>(k[4]) : 0.0f;
 }
 
-// Level-1 operator: per search cell, the bins of its rows in order.
+// Level-1 operator: per search cell, the bins of its rows in order, and the cell's weight in
+// the single-launch loop's split: a row's vector work counts like about 30 of its entries.
+constexpr int kRowWork = 30;
+
 __global__ void k_mg_cells(MgLevel L1, const int32_t* cell_start, const double* bins, int n, float omega,
-                           const DevStatus* status, int32_t* active_flag) {
+                           const DevStatus* status, int32_t* active_flag, const int32_t* len, int32_t* cell_w) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= L1.cells) return;
     const int b = cell_start[c], e = cell_start[c + 1];
@@ -118,10 +121,13 @@ __global__ void k_mg_cells(MgLevel L1, const int32_t* cell_start, const double* 
     double k[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) k[q] = 0.0;
+    int work = 0;
     for (int i = b; i < e; i++) {
 #pragma unroll
         for (int q = 0; q < 9; q++) k[q] += bins[static_cast<int64_t>(q) * n + i];
+        work += len[i] + kRowWork;
     }
+    cell_w[c] = work;
     store_level(L1, c, k, omega);
 }
 
@@ -904,16 +910,19 @@ cudaError_t mg_prepare_device() {
     const int dense_max = (2 * kMgDenseCells * kMgDenseCells + kMgDenseCells) * static_cast<int>(sizeof(float));
     cudaError_t e = cudaFuncSetAttribute(k_mg_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, dense_max);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(kMgBottomBytes));
+    e = cudaFuncSetAttribute(k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kMgBottomBytes));
+    if (e != cudaSuccess) return e;
+    return pcg_loop_prepare_device();
 }
 
-void mg_setup_level1(const MgHierarchy& mg, const CgOperands& o, cudaStream_t s) {
+void mg_setup_level1(const MgHierarchy& mg, const CgOperands& o, cudaStream_t s, bool lists) {
     // cells without particles keep a zero residual through the solve
     cudaMemsetAsync(mg.lv[1].r, 0, sizeof(float) * mg.lv[1].cells, s);
     k_mg_bins<<<o.grid_spmv, kBlock, 0, s>>>(o, mg.cell_xz, mg.bins, mg.dinv0, kMgOmegaFine, mg.status);
     k_mg_cells<<<grid_for(mg.lv[1].cells), kBlock, 0, s>>>(mg.lv[1], mg.cell_start, mg.bins, mg.n,
-                                                          kMgOmegaCoarse, mg.status, mg.active_flag);
+                                                          kMgOmegaCoarse, mg.status, mg.active_flag, o.len, mg.cell_w);
+    if (!lists) return;
     launch_exclusive_scan(mg.active_flag, mg.active_pos, mg.lv[1].cells, mg.scan_scratch, s);
     k_mg_active<<<grid_for(mg.lv[1].cells), kBlock, 0, s>>>(mg.lv[1].cells, mg.active_flag, mg.active_pos,
                                                            mg.cell_start, mg.active, mg.active_rows);
@@ -931,7 +940,7 @@ void mg_setup(const MgHierarchy& mg, const CgOperands& o, cudaStream_t s) {
     mg_setup_coarse(mg, s);
 }
 
-int mg_setup_launches(const MgHierarchy& mg) { return 2 + 3 + 1 + (mg.levels - 1) + 1; }
+int mg_setup_launches(const MgHierarchy& mg, bool lists) { return 2 + (lists ? 4 : 0) + (mg.levels - 1) + 1; }
 
 void mg_apply(const MgHierarchy& mg, const CgScalars* S, int mode, const float* r, float* u,
               cudaStream_t s, const CgOperands* fuse_axpy) {

@@ -71,8 +71,15 @@ struct MgHierarchy {
     int32_t* active_flag = nullptr;     // per level-1 cell: 1 with particles
     int32_t* active_pos = nullptr;      // exclusive prefix sum of active_flag (cells + 1)
     int32_t* scan_scratch = nullptr;
+    int32_t* cell_w = nullptr;          // per level-1 cell: its rows' work in the single-launch loop
     DevStatus* status = nullptr;
 };
+
+// pcgloop.cu: the preconditioned iteration loop in one launch (after mg_setup and k_mx_init).
+// It writes the solution into x (no k_mx_finish after it).
+bool pcg_loop_fits(const MgHierarchy& mg);
+cudaError_t launch_pcg_loop(const CgOperands& o, const MgHierarchy& mg, cudaStream_t s);
+cudaError_t pcg_loop_prepare_device();
 
 // Level sizes for a gnx x gnz search grid (returns the level count, 0 if the grid is
 // too large for the 16-bit cell coordinates or the level count).
@@ -83,9 +90,10 @@ void mg_setup(const MgHierarchy& mg, const CgOperands& o, cudaStream_t s);
 // The two halves of mg_setup: the level-1 operator (reads the matrix), then the coarser
 // Galerkin operators and the dense inverse (read only the level-1 operator), which can
 // run beside other work that does not use the hierarchy.
-void mg_setup_level1(const MgHierarchy& mg, const CgOperands& o, cudaStream_t s);
+// (lists: with the list of cells that hold rows, which the per-phase cycle kernels walk)
+void mg_setup_level1(const MgHierarchy& mg, const CgOperands& o, cudaStream_t s, bool lists = true);
 void mg_setup_coarse(const MgHierarchy& mg, cudaStream_t s);
-int mg_setup_launches(const MgHierarchy& mg);
+int mg_setup_launches(const MgHierarchy& mg, bool lists = true);
 // u = M r.  `mode` gates the kernels on the solve state like the PCG kernels: 0 init,
 // 1 iteration, 2 after a reliable update (see pcg_skip).  With `fuse_axpy` (mode 1) the
 // iteration's vector updates run in the restriction kernel, which then produces r.

@@ -456,6 +456,7 @@ void allocate(mps_handle* h, int64_t n, int64_t keep) {
         mg.active = dalloc<int32_t>(h, mg.lv[1].cells);
         mg.active_rows = dalloc<int2>(h, mg.lv[1].cells);
         mg.active_flag = dalloc<int32_t>(h, mg.lv[1].cells);
+        mg.cell_w = dalloc<int32_t>(h, mg.lv[1].cells);
         mg.active_pos = dalloc<int32_t>(h, mg.lv[1].cells + 1);
         mg.n_active = mg.active_pos + mg.lv[1].cells;
         mg.scan_scratch = dalloc<int32_t>(h, scan_scratch_ints(mg.lv[1].cells));
@@ -635,12 +636,6 @@ int default_max_iter(int32_t requested, int64_t n, int32_t solver) {
     return static_cast<int>(std::min<int64_t>(lim, 0x7fffffff));
 }
 
-// Kernels of a plain solve's graph: init (and MIXED's first SpMV), the loop, [finish], with
-// a fallback its init, loop and merge, the true residual.
-int plain_solve_launches(int solver, bool with_fb) {
-    return solver == MPS_SOLVER_CG64 ? 3 : 5 + (with_fb ? 3 : 0);
-}
-
 void after_launch(const char* what) { check(cudaGetLastError(), what); }
 
 // Reads the status block and converts device flags into the reference's errors.
@@ -677,17 +672,15 @@ void read_status(mps_handle* h, bool solve_done) {
         h->stats.cg_true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
         if (h->direct_launches >= 0) {
             launched(h, static_cast<int>(h->direct_launches));
-        } else if (h->prm.solver == MPS_SOLVER_CG64) {
-            launched(h, plain_solve_launches(MPS_SOLVER_CG64, false));
-        } else if (is_preconditioned(h->prm.solver)) {
+        } else if (h->cg.one_launch()) {
+            launched(h, one_launch_count(h->prm.solver, &h->mg, h->prm.solver != MPS_SOLVER_CG64));
+        } else {
             const int kpi = h->cg.kernels_per_iteration(), kpu = h->cg.kernels_per_update();
             const int own = S.iter - S.fb_iter;
             // per-phase kernels and the finish kernel, or one persistent kernel
             const int loop = h->cg.persistent() ? 1 : own * kpi + S.updates * kpu + 1;
             launched(h, mg_setup_launches(h->mg) + 2 + mg_apply_launches(h->mg) + loop + 4 +
                             (h->prm.solver == MPS_SOLVER_LEARNED ? 1 + learned_prep_launches(h->mg, true) : 0));
-        } else {
-            launched(h, plain_solve_launches(h->prm.solver, true));
         }
     }
     const int f = h->h_status->flags;
@@ -2006,7 +1999,7 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         check(cudaStreamSynchronize(s), "cg solve");
         if (iterations) *iterations = S.iter;
         if (true_relres) *true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
-        h->stats.kernel_launches += 1 + plain_solve_launches(solver, false);
+        h->stats.kernel_launches += 1 + one_launch_count(solver, nullptr, false);
         if (!S.converged)
             throw StatusError{MPS_ERR_CG_NOT_CONVERGED,
                               "Conjugate Gradient method couldn't solve Pressure Poison Equation"};
