@@ -20,10 +20,11 @@ namespace mpsgb {
 
 namespace {
 
-constexpr int kPartUnits = 320;  // unit sums of a tile (80 KB of doubles)
-constexpr int kTileChunks = kPartUnits / kMaxUnits;
+constexpr int kTileChunks = 128;  // of a block whose chunks pass the tables
 
-// dynamic shared memory: unit sums, chunk table, unit table, vectors
+// dynamic shared memory: unit sums, tables, vectors.  (The gathered vector's rows around the
+// block in shared memory too were measured: 42,226 rows 13.0 against 12.4 us, 90,050 rows
+// 18.8 against 18.4, MIXED 13.9 against 14.0: loading them costs what the gathers wait.)
 struct LoopPlan {
     int blocks;
     int tables;      // chunks the tables hold: all that a block can own, or one tile
@@ -32,7 +33,7 @@ struct LoopPlan {
 };
 
 size_t table_bytes(int tables) {
-    return sizeof(double) * kPartUnits * 32 + static_cast<size_t>(kChunkBytes) * tables;
+    return part_room(tables) + table_room(tables);
 }
 
 // This block's chunks.  o.loop_w[c] is the width of a chunk the loop works on, 0 for one it
@@ -46,8 +47,7 @@ __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPla
     LoopView L;
     L.lo = 0;
     L.hi = o.n;
-    L.part = reinterpret_cast<double*>(sm);
-    *keep = place_tables(L, L.part + kPartUnits * 32, plan.tables);
+    *keep = place_tables(L, sm, plan.tables);
     const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x), lane = t & 31;
     L.warps = nt >> 5;
     const int seg = (o.nchunks + nt - 1) / nt;
@@ -113,7 +113,7 @@ __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPla
             L.nc = L.whole ? mine : last_chunk - first_chunk + 1;
         }
     }
-    split_tiles(L, kPartUnits, plan.tables);
+    split_tiles(L, plan.tables);
     if (L.whole) build_tables(o, L, L.nc);
     return L;
 }
@@ -359,10 +359,10 @@ size_t g_loop_smem = 0;    // largest dynamic shared memory of a block
 // SMs have a tenth of the FP64 pipes and of the loads in flight.  us per iteration, cluster
 // against grid (dam breaks at r_e = 4 l0; the WHILE node's kernels took 29-31 and 19-21):
 //   rows      1,850        3,133        5,250         9,403
-//   CG64    6.4 / 8.2    8.7 / 8.0   11.2 / 8.1    16.8 / 8.6
-//   MIXED   5.5 / 7.1    6.1 / 7.3    8.2 / 7.1    11.1 / 7.1
-// The grid form at 16,850, 42,226, 90,050 and 340,050 rows: CG64 9.7, 13.5, 21.9, 58.0
-// (WHILE: 30.4, 31.5, 37.2, 73.7), MIXED 8.0, 9.4, 16.4 (20.6, 21.7, 25.1); the FP64 pipe
+//   CG64    6.2 / 8.2    8.7 / 7.9   11.2 / 8.0    16.8 / 8.5
+//   MIXED   5.4 / 7.1    5.8 / 7.3    8.2 / 7.2    11.1 / 7.2
+// The grid form at 16,850, 42,226, 90,050 and 340,050 rows: CG64 9.4, 12.4, 18.4, 52.0
+// (WHILE: 30.4, 31.5, 37.2, 73.7), MIXED 7.7, 9.4, 14.0 (20.6, 21.7, 25.1); the FP64 pipe
 // bounds the large CG64 systems (one multiply-add per entry: 6.4 us at 90,050 rows), the
 // exchanges the small ones.
 constexpr int kClusterChunks64 = 80, kClusterChunks32 = 128;
@@ -371,12 +371,16 @@ LoopPlan loop_plan(int nchunks, bool cluster, int keep_row_bytes) {
     LoopPlan p{};
     p.blocks = cluster ? g_loop_cluster : g_loop_sms;
     if (!cluster && p.blocks > nchunks) p.blocks = nchunks;
-    const int most = 5 * ((nchunks + p.blocks - 1) / p.blocks) + 2;
-    p.tables = table_bytes(most) <= g_loop_smem ? most : kTileChunks;
-    const size_t room = g_loop_smem - table_bytes(p.tables);
+    const int per = (nchunks + p.blocks - 1) / p.blocks;
+    p.tables = kTileChunks;
+    if (table_bytes(3 * per + 2) <= g_loop_smem / 2)
+        p.tables = 3 * per + 2;
+    else if (table_bytes(2 * per + 2) <= g_loop_smem / 4 * 3)
+        p.tables = 2 * per + 2;
+    const size_t left = g_loop_smem - table_bytes(p.tables);
     // half as much again as the average block's vectors (the rest of the SM's memory is L1)
-    const size_t want = (static_cast<size_t>(nchunks) * 3 / (2 * p.blocks) + 4) * kSellRows * keep_row_bytes;
-    p.keep_bytes = static_cast<int>(want < room ? want : room);
+    const size_t want = (static_cast<size_t>(per) * 3 / 2 + 4) * kSellRows * keep_row_bytes;
+    p.keep_bytes = static_cast<int>(want < left ? want : left);
     p.smem = table_bytes(p.tables) + p.keep_bytes;
     return p;
 }

@@ -1,11 +1,12 @@
 // cgloop.cuh - the matrix products of the single-launch solver loops (cgloop.cu, pcgloop.cu).
 //
-// A block owns a range of SELL chunks.  For a product A v they are cut into units of a few
-// entries of a chunk's 32 rows (one warp per unit, one lane per row), the unit sums are
-// parked in shared memory and the row's thread adds them: with whole chunks per warp, 17
-// chunks of 46 entries (84k rows over 152 SMs) would occupy 17 of 32 warps, and a 58-chunk
-// system (1,850 rows) would wait for one lane's 46 dependent multiply-adds.  Blocks with
-// more chunks than the sums' room take them in tiles.
+// A block owns a range of SELL chunks.  A product A v reads them in steps of eight entries of
+// a chunk's 32 rows, one lane per row; the block's steps, chunk after chunk, are dealt to its
+// warps in equal contiguous shares.  A unit is the part of one chunk in one warp's share: its
+// sums are parked in shared memory and the row's thread adds them.  18 chunks of 41 entries
+// (84k rows over 152 SMs) are 108 steps, seven for each of 16 warps at most; in units of 16
+// entries dealt out whole (MIXED 16.4, CG64 21.9 us an iteration at 90,050 rows) the longest
+// warp had ten.  Blocks with more chunks than the tables hold take them in tiles.
 #pragma once
 
 #include "cg.cuh"
@@ -16,98 +17,113 @@ namespace mpsgb {
 namespace {
 
 constexpr int kStep = 8;         // matrix entries a lane loads at once
-constexpr int kMaxUnits = 8;     // units of one chunk (longer rows take longer units)
-// Units a warp should have: with two, 18 chunks (84k rows over 152 SMs) are 36 units for 16
-// warps and the last round is nearly empty.  us per iteration at two, three, four, six:
-// CG64 23.4, 21.5, 21.9, 21.9 and MIXED 17.5, 15.9, 16.4, 16.4 at 90,050 rows; MIXED 20.2,
-// 19.1, 18.5, 18.3 on a 3D dam break of 210,868 particles.
-constexpr int kUnitsPerWarp = 4;
 
 struct __align__(16) ChunkInfo {
-    int chunk, off, width, span;  // span: entries of a unit
-    int first, units;             // its first unit
-    unsigned live;                // rows of the block with entries
-    int pad;
+    int chunk, off, width, steps;
+    int first, units;  // its first unit
+    unsigned live;     // rows of the block with entries
+    int before;        // steps of the chunks before it
 };
 
-// Shared memory of a table's chunk.
-constexpr int kChunkBytes = static_cast<int>(sizeof(ChunkInfo) + sizeof(int2) * kMaxUnits);
-
 struct LoopView {
-    double* part;     // unit sums, `part_units` x 32
+    double* part;     // unit sums, `parts` x 32
     ChunkInfo* info;  // all chunks of the block (whole) or those of a tile
-    int2* unit;       // {table index, first entry}, kMaxUnits per chunk
+    int4* unit;       // {table index, first entry, end}
+    int2* share;      // per warp: its first unit and end
     int c0, nc;  // whole: table entries are the chunks; else chunks c0 .. c0 + nc - 1
     int lo, hi;  // rows of the block (its first and last chunk may hold others' rows)
     int tile;    // chunks per tile
     int active;  // threads that own rows
     int warps;
-    int cuts;  // units of a chunk, at most kMaxUnits
     bool whole;
 };
 
-// Entries of a unit of a chunk `width` entries wide.  A block with chunks to spare takes
-// them in few units (each unit past the first costs the row an addition); one with few
-// cuts them so that its warps all have one.
-__device__ __forceinline__ int unit_span(const LoopView& L, int width) {
-    const int per = (width + L.cuts - 1) / L.cuts;
-    return (per + kStep - 1) / kStep * kStep;
+// Shared memory of the tables of `tables` chunks: ChunkInfo and units (each chunk's last is
+// its own or shared with a warp's end, so there are at most chunks + warps), shares.
+__host__ __device__ constexpr size_t table_room(int tables) {
+    return sizeof(ChunkInfo) * static_cast<size_t>(tables) +
+           sizeof(int4) * static_cast<size_t>(tables + kLoopThreads / 32) + sizeof(int2) * (kLoopThreads / 32);
+}
+// and of their unit sums
+__host__ __device__ constexpr size_t part_room(int tables) {
+    return sizeof(double) * 32 * static_cast<size_t>(tables + kLoopThreads / 32);
 }
 
-// Lays the tables of `tables` chunks out at `at`; returns their end.
+// Lays unit sums and tables of `tables` chunks out at `at`; returns their end.
 __device__ __forceinline__ unsigned char* place_tables(LoopView& L, void* at, int tables) {
-    L.info = static_cast<ChunkInfo*>(at);
-    L.unit = reinterpret_cast<int2*>(L.info + tables);
-    return reinterpret_cast<unsigned char*>(L.unit + static_cast<size_t>(tables) * kMaxUnits);
+    L.part = static_cast<double*>(at);
+    L.info = reinterpret_cast<ChunkInfo*>(static_cast<unsigned char*>(at) + part_room(tables));
+    L.unit = reinterpret_cast<int4*>(L.info + tables);
+    L.share = reinterpret_cast<int2*>(L.unit + tables + kLoopThreads / 32);
+    return reinterpret_cast<unsigned char*>(L.share + kLoopThreads / 32);
 }
 
 // Completes the table entries [0, m) whose chunks are set, and lists their units.
 __device__ __forceinline__ void build_tables(const CgOperands& o, const LoopView& L, int m) {
     const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
+    const long long W = L.warps;
     for (int k = t; k < m; k += nt) {
         const int c = L.info[k].chunk;
         const int w = o.chunk[c] / kSellRows;
         L.info[k].off = o.off[c];
         L.info[k].width = w;
-        L.info[k].span = unit_span(L, w);
-        L.info[k].units = w > 0 ? (w + L.info[k].span - 1) / L.info[k].span : 0;
+        L.info[k].steps = (w + kStep - 1) / kStep;
     }
     for (int k = t >> 5; k < m; k += nt >> 5) {
         const int row = L.info[k].chunk * kSellRows + (t & 31);
         const unsigned live = __ballot_sync(0xffffffffu, row >= L.lo && row < L.hi && o.len[row] > 0);
         if ((t & 31) == 0) L.info[k].live = live;
     }
+    if (t < L.warps) L.share[t] = make_int2(0, 0);
+    __shared__ int steps;
     __syncthreads();
-    if (t < 32) {  // exclusive prefix sum of the unit counts
+    // exclusive prefix sums over the table, by one warp
+    auto scan = [&](auto value, auto store) {
         int run = 0;
         for (int b = 0; b < m; b += 32) {
-            const int u = b + t < m ? L.info[b + t].units : 0;
+            const int u = b + t < m ? value(L.info[b + t]) : 0;
             int s = u;
             for (int d = 1; d < 32; d <<= 1) {
                 const int x = __shfl_up_sync(0xffffffffu, s, d);
                 if (t >= d) s += x;
             }
-            if (b + t < m) L.info[b + t].first = run + s - u;
+            if (b + t < m) store(L.info[b + t], run + s - u);
             run += __shfl_sync(0xffffffffu, s, 31);
         }
+        return run;
+    };
+    if (t < 32) {
+        const int T = scan([](const ChunkInfo& c) { return c.steps; }, [](ChunkInfo& c, int x) { c.before = x; });
+        if (t == 0) steps = T;
+        __syncwarp();
+        scan(
+            [&](ChunkInfo& c) {
+                if (c.steps == 0) return c.units = 0;
+                if (T < W) return c.units = c.steps;
+                return c.units = static_cast<int>((c.before + c.steps - 1) * W / T - c.before * W / T) + 1;
+            },
+            [](ChunkInfo& c, int x) { c.first = x; });
     }
     __syncthreads();
+    const int T = steps;  // step s is warp floor(s W / T)'s, whose first is start(warp)
+    auto start = [&](int v) { return static_cast<int>((static_cast<long long>(v) * T + W - 1) / W); };
     for (int k = t; k < m; k += nt) {
         const ChunkInfo c = L.info[k];
-        for (int u = 0; u < c.units; u++) L.unit[c.first + u] = make_int2(k, u * c.span);
+        for (int u = 0; u < c.units; u++) {
+            const int v = static_cast<int>((c.before + (T < W ? u : 0)) * W / T) + (T < W ? 0 : u);
+            const int a = start(v), b = start(v + 1);
+            const int s0 = max(c.before, a), s1 = min(c.before + c.steps, b);
+            L.unit[c.first + u] = make_int4(k, (s0 - c.before) * kStep, min(c.width, (s1 - c.before) * kStep), 0);
+            if (s0 == a) L.share[v].x = c.first + u;
+            if (s1 == b) L.share[v].y = c.first + u + 1;
+        }
     }
     __syncthreads();
 }
 
-// Tiles and cuts of a block with L.nc chunks whose unit sums have room for part_units and
-// whose tables hold `tables` chunks.
-__device__ __forceinline__ void split_tiles(LoopView& L, int part_units, int tables) {
-    const int nc = max(1, L.nc);
-    const int cuts = min(kMaxUnits, (kUnitsPerWarp * L.warps + nc - 1) / nc);
-    int tiles = (nc * cuts + part_units - 1) / part_units;
-    if (!L.whole) tiles = max(tiles, (nc + tables - 1) / tables);
-    L.tile = (nc + tiles - 1) / tiles;
-    L.cuts = min(min(kMaxUnits, (kUnitsPerWarp * L.warps + L.tile - 1) / L.tile), part_units / L.tile);
+// Tiles of a block with L.nc chunks whose tables hold `tables` chunks.
+__device__ __forceinline__ void split_tiles(LoopView& L, int tables) {
+    L.tile = L.whole ? max(1, L.nc) : tables;
     L.active = min(static_cast<int>(blockDim.x), L.nc * 32);
 }
 
@@ -146,13 +162,13 @@ struct UnitCursor {
     int64_t at;  // the lane's first entry of the chunk
 
     __device__ __forceinline__ void open() {
-        const int2 un = L.unit[u];
+        const int4 un = L.unit[u];
         const int lane = threadIdx.x & 31;
         const ChunkInfo& ci = L.info[un.x];
         at = static_cast<int64_t>(ci.off) + lane;
         row = ci.chunk * kSellRows + lane;
         k0 = un.y;
-        end = min(ci.width, k0 + ci.span);
+        end = un.z;
         live = (ci.live >> lane & 1u) != 0u;
     }
     __device__ __forceinline__ UnitCursor(const CgOperands& o_, const LoopView& L_, int u_, int u1_)
@@ -188,23 +204,21 @@ struct UnitCursor {
         }
         k0 += kStep;
         if (k0 >= end) {
-            s.out = u;
-            u += L.warps;
+            s.out = u++;
             if (u < u1) open();
         }
     }
 };
 
-// Unit sums of table chunks [a, b): T = double (FP64 matrix) or float (FP32 pairs).  Two
+// The unit sums of the tables' chunks: T = double (FP64 matrix) or float (FP32 pairs).  Two
 // steps in turn, each loaded while the other gathers and adds: a warp waits for one round
-// trip to L2 per step (0.6 us across the dies), not for two.  Unit u's sums go to place
-// u - base.
+// trip to L2 per step (0.6 us across the dies), not for two.
 template <class T, class V>
-__device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L, int a, int b, int base, V v) {
+__device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L, V v) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     T* part = reinterpret_cast<T*>(L.part);
-    const int u0 = L.info[a].first, u1 = L.info[b - 1].first + L.info[b - 1].units;
-    UnitCursor<T> cur(o, L, u0 + warp, u1);
+    const int2 mine = L.share[warp];
+    UnitCursor<T> cur(o, L, mine.x, mine.y);
     if (!cur.valid()) return;
     T acc = 0;
     auto add = [&](const UnitStep<T>& s) {
@@ -219,7 +233,7 @@ __device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L
             }
         }
         if (s.out >= 0) {
-            part[(s.out - base) * 32 + lane] = acc;
+            part[s.out * 32 + lane] = acc;
             acc = 0;
         }
     };
@@ -252,13 +266,12 @@ __device__ __forceinline__ void product(const CgOperands& o, const LoopView& L, 
             __syncthreads();
             build_tables(o, L, k1 - k0);
         }
-        const int u0 = L.info[k0 - table0].first;
-        unit_sums<T>(o, L, k0 - table0, k1 - table0, u0, v);
+        unit_sums<T>(o, L, v);
         __syncthreads();
         const int skip = k0 % L.warps;  // chunk k belongs to warp k % warps
         for (int k = k0 - skip + warp + (warp < skip ? L.warps : 0); k < k1; k += L.warps) {
             const ChunkInfo c = L.info[k - table0];
-            const T* p = part + (c.first - u0) * 32 + lane;
+            const T* p = part + c.first * 32 + lane;
             T s = c.units > 0 ? p[0] : T(0);  // two chains of additions
             if (c.units > 1) {
                 T q = p[32];

@@ -21,10 +21,10 @@
 // us per solve, the chain against this loop (GB300, dam breaks at r_e = 4 l0):
 //   rows       1,850   3,133   5,250   9,403  16,850  42,226  90,050   hydrostatic 84,450
 //   chain      1,684   1,861   1,882   2,087   2,075   2,752   2,896   2,634
-//   loop         760     936   1,018   1,172   1,174   1,676   2,450   1,900
+//   loop         742     936   1,004   1,156   1,154   1,637   2,419   1,855
 // An iteration's bound is latency: at 1,850 rows 5,000 of 24,000 cycles are the bottom
 // levels' chain of shared-memory steps, 6,900 the sum and its divisions, 3,300 the SpMV's
-// four dependent steps; at 84k rows 13,000 of 55,000 are the SpMV (28 MB from L2, which
+// four dependent steps; at 84k rows 11,000 of 53,000 are the SpMV (28 MB from L2, which
 // alone would stream in 4,000), 11,000 the sum, 10,000 the bottom levels.  340,050 rows do
 // not fit (window, own vectors and bottom levels pass the SM's shared memory): the chain.
 #include <algorithm>
@@ -36,8 +36,6 @@
 namespace mpsgb {
 
 namespace {
-
-constexpr int kPcgParts = 128;  // unit sums of a tile
 
 // Sizes of the dynamic shared memory: bottom levels, unit sums, tables, own rows, window,
 // cells around.
@@ -172,13 +170,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
         }
     }
     __syncthreads();
-    const int span_rows = rg.before[2] + rg.rb[2] - rg.ra[2];
 
     // ---- shared memory
     float* bot = pcg_sm;
-    double* part = reinterpret_cast<double*>(bot + plan.bottom_floats);
     LoopView V;
-    float* own = reinterpret_cast<float*>(place_tables(V, part + kPcgParts * 32, plan.tables));
+    float* own = reinterpret_cast<float*>(place_tables(V, bot + plan.bottom_floats, plan.tables));
     ChunkInfo* const info = V.info;
     float* win_u = own + 5 * static_cast<size_t>(plan.rows);
     float* win_d = win_u + plan.window;
@@ -241,14 +237,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
     // the own rows' vectors, kept (index: row - r0) or global (index: row)
     const bool keep = rows <= plan.rows;
     if (t == 0) {
-        V.part = part;
         V.warps = nt >> 5;
         V.lo = r0;
         V.hi = r1;
         V.c0 = r0 / kSellRows;
         V.nc = rows > 0 ? (r1 - 1) / kSellRows - V.c0 + 1 : 0;
         V.whole = V.nc <= plan.tables;
-        split_tiles(V, kPcgParts, plan.tables);
+        split_tiles(V, plan.tables);
         L = V;
         float* const global[5] = {o.s32, o.p32, o.d32, o.w32, o.r32};
         for (int k = 0; k < 5; k++) vec[k] = keep ? own + k * plan.rows - r0 : global[k];
@@ -568,8 +563,7 @@ bool pcg_plan(const MgHierarchy& mg, bool cluster, PcgPlan* plan) {
     if (p.window > mg.n + 4) p.window = (mg.n + 3) & ~3;
     if (p.window > 65532) p.window = 65532;
     p.cells = (p.window / 4 + 3) & ~3;
-    const size_t fixed = sizeof(double) * kPcgParts * 32 +
-                         static_cast<size_t>(kChunkBytes) * p.tables +
+    const size_t fixed = part_room(p.tables) + table_room(p.tables) +
                          static_cast<size_t>(kRowBytes) * p.rows + static_cast<size_t>(kWindowBytes) * p.window +
                          static_cast<size_t>(kCellBytes) * p.cells;
     for (p.bottom = mg.bottom; p.bottom <= mg.levels; p.bottom++) {
