@@ -59,9 +59,12 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     return v;
 }
 
-// Block sums of three values, the same in every thread (warp partials in order).
+// Block sums of three values, the same in every thread (warp partials in order).  One thread
+// per value adds the partials: an FP64 addition takes a scheduler's pipe 64 cycles a warp, so
+// the same 96 additions in every warp of a 1024-thread block took 49,000 cycles.
 template <int T>
 __device__ void block_sum3(double& a, double& b, double& c, double* red) {
+    __shared__ double total[3];
     a = warp_sum_d(a);
     b = warp_sum_d(b);
     c = warp_sum_d(c);
@@ -72,16 +75,15 @@ __device__ void block_sum3(double& a, double& b, double& c, double* red) {
         red[64 + w] = c;
     }
     __syncthreads();
-    double x = 0.0, y = 0.0, z = 0.0;
-    for (int k = 0; k < T / 32; k++) {
-        x += red[k];
-        y += red[32 + k];
-        z += red[64 + k];
+    if (threadIdx.x < 3) {
+        double x = 0.0;
+        for (int k = 0; k < T / 32; k++) x += red[32 * threadIdx.x + k];
+        total[threadIdx.x] = x;
     }
     __syncthreads();
-    a = x;
-    b = y;
-    c = z;
+    a = total[0];
+    b = total[1];
+    c = total[2];
 }
 
 __device__ __forceinline__ bool step_failed_batch(const DevStatus* st) {
@@ -103,17 +105,29 @@ __device__ void setup_scene(const BatchOps& B, const Smem& S, const BatchScene& 
         if (ci >= 0) {
             const int L = o.len[i];
             int64_t at = sell_index(o.off[i >> 5], lane, 0);
-            for (int k = 0; k < L; k++, at += kSellRows) {
-                const int j = o.col[at];
-                const double a = o.val[at];
-                if (j == i) aii = a;
-                const int cj = B.cell_xz[j];
+            for (int k0 = 0; k0 < L; k0 += 4, at += 4 * kSellRows) {
+              int jj[4], cc[4];
+              double aa[4];
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                jj[u] = k0 + u < L ? __ldcs(o.col + at + u * kSellRows) : i;
+                aa[u] = k0 + u < L ? __ldcs(o.val + at + u * kSellRows) : 0.0;
+              }
+#pragma unroll
+              for (int u = 0; u < 4; u++) cc[u] = B.cell_xz[jj[u]];
+#pragma unroll
+              for (int v = 0; v < 4; v++) {
+                if (k0 + v >= L) break;
+                const double a = aa[v];
+                if (jj[v] == i) aii = a;
+                const int cj = cc[v];
                 const int dx = (cj >> 16) - (ci >> 16), dz = (cj & 0xffff) - (ci & 0xffff);
                 const bool ok = cj >= 0 && dx >= -1 && dx <= 1 && dz >= -1 && dz <= 1;
                 const int q = (dx + 1) * 3 + dz + 1;
                 const float af = static_cast<float>(a);
 #pragma unroll
                 for (int u = 0; u < 9; u++) b9[u] += (ok && u == q) ? af : 0.0f;
+              }
             }
         }
         const bool active = ci >= 0 && aii < 0.0;
@@ -232,7 +246,17 @@ __device__ void apply_m(const BatchOps& B, const Smem& S, const BatchScene& sc, 
         const int cnt = min(B.cell_count[cellbase + c], B.max_per_cell);
         const int32_t* slots = B.cell_slot + static_cast<int64_t>(cellbase + c) * B.max_per_cell;
         float sum = 0.0f;
-        for (int s = 0; s < cnt; s++) sum += o.r32[slots[s]];
+        for (int s = 0; s < cnt; s += 4) {
+            int i[4];
+            float x[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) i[u] = s + u < cnt ? slots[s + u] : 0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = s + u < cnt ? o.r32[i[u]] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (s + u < cnt) sum += x[u];
+        }
         S.r[1][c] = sum;
     }
     __syncthreads();
@@ -272,6 +296,59 @@ __device__ void apply_m(const BatchOps& B, const Smem& S, const BatchScene& sc, 
     __syncthreads();
 }
 
+// Entries of a row a lane loads before it gathers and adds them: a block has its SM to
+// itself or shares it with one other, so each lane has to keep several round trips in
+// flight.  The sums are those of one entry at a time.
+constexpr int kRowStep32 = 8, kRowStep64 = 4;
+
+__device__ __forceinline__ float batch_row32(const CgOperands& o, int i, const float* v) {
+    constexpr int D = kRowStep32;
+    const int L = o.len[i];
+    const uint2* cv = o.cv32 + sell_index(o.off[i >> 5], i & 31, 0);
+    float acc = 0.0f;
+    uint2 e[D];
+#pragma unroll
+    for (int u = 0; u < D; u++) e[u] = u < L ? ld_sell_pair(cv + u * kSellRows) : make_uint2(0u, 0u);
+    for (int k = 0; k < L; k += D) {
+        float x[D], a[D];
+#pragma unroll
+        for (int u = 0; u < D; u++) x[u] = k + u < L ? v[e[u].x] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < D; u++) a[u] = __uint_as_float(e[u].y);
+        cv += D * kSellRows;
+#pragma unroll
+        for (int u = 0; u < D; u++) e[u] = k + D + u < L ? ld_sell_pair(cv + u * kSellRows) : make_uint2(0u, 0u);
+#pragma unroll
+        for (int u = 0; u < D; u++)
+            if (k + u < L) acc = fmaf(a[u], x[u], acc);
+    }
+    return acc;
+}
+
+__device__ __forceinline__ double batch_row64(const CgOperands& o, int i, const double* v) {
+    constexpr int D = kRowStep64;
+    const int L = o.len[i];
+    const int64_t at = sell_index(o.off[i >> 5], i & 31, 0);
+    const int32_t* col = o.col + at;
+    const double* val = o.val + at;
+    double acc = 0.0;
+    for (int k = 0; k < L; k += D, col += D * kSellRows, val += D * kSellRows) {
+        int c[D];
+        double a[D], x[D];
+#pragma unroll
+        for (int u = 0; u < D; u++) {
+            c[u] = k + u < L ? __ldcs(col + u * kSellRows) : 0;
+            a[u] = k + u < L ? __ldcs(val + u * kSellRows) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < D; u++) x[u] = k + u < L ? v[c[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < D; u++)
+            if (k + u < L) acc = fma(a[u], x[u], acc);
+    }
+    return acc;
+}
+
 // w = A u (FP32 matrix); returns gamma = r.u, delta = w.u, rho = r.r (FP64 sums)
 template <int T>
 __device__ void spmv_dots(const BatchOps& B, const Smem& S, const BatchScene& sc, double& gam, double& del,
@@ -280,17 +357,11 @@ __device__ void spmv_dots(const BatchOps& B, const Smem& S, const BatchScene& sc
     double g = 0.0, d = 0.0, r = 0.0;
     for (int t = threadIdx.x; t < sc.rows; t += T) {
         const int i = sc.row0 + t;
-        const int L = o.len[i];
-        int64_t at = sell_index(o.off[i >> 5], i & 31, 0);
-        float acc = 0.0f;
-        for (int k = 0; k < L; k++, at += kSellRows) {
-            const uint2 e = ld_sell_pair(o.cv32 + at);
-            acc = fmaf(__uint_as_float(e.y), o.u32[e.x], acc);
-        }
+        const float acc = batch_row32(o, i, o.u32);
         o.w32[i] = acc;
-        const double ri = o.r32[i], ui = o.u32[i];
+        const double ri = widen(o.r32[i]), ui = widen(o.u32[i]);
         g += ri * ui;
-        d += static_cast<double>(acc) * ui;
+        d += widen(acc) * ui;
         r += ri * ri;
     }
     block_sum3<T>(g, d, r, S.red);
@@ -307,10 +378,7 @@ __device__ void residual64(const BatchOps& B, const Smem& S, const BatchScene& s
     double a = 0.0, b = 0.0, z = 0.0;
     for (int t = threadIdx.x; t < sc.rows; t += T) {
         const int i = sc.row0 + t;
-        const int L = o.len[i];
-        int64_t at = sell_index(o.off[i >> 5], i & 31, 0);
-        double acc = 0.0;
-        for (int k = 0; k < L; k++, at += kSellRows) acc = fma(o.val[at], o.x[o.col[at]], acc);
+        const double acc = batch_row64(o, i, o.x);
         const double ri = o.b[i] - acc;
         o.r32[i] = static_cast<float>(ri);
         if (to64) {
@@ -400,8 +468,15 @@ __device__ void solve_scene(const BatchOps& B, const Smem& S, int k) {
                 apply_m<T>(B, S, sc, cellbase);
                 spmv_dots<T>(B, S, sc, gam, del, rho);
             }
-            beta = gam / gam_old;
-            alpha = gam / (del - beta * gam / alpha);
+            // one thread's divisions: in every warp they took 14,000 cycles
+            __shared__ double step[2];
+            if (threadIdx.x == 0) {
+                step[0] = gam / gam_old;
+                step[1] = gam / (del - step[0] * gam / alpha);
+            }
+            __syncthreads();
+            beta = step[0];
+            alpha = step[1];
             gam_old = gam;
             iter++;
             if (!(std::isfinite(alpha) && std::isfinite(beta) && alpha != 0.0)) stalled = true;
@@ -428,10 +503,7 @@ __device__ void solve_scene(const BatchOps& B, const Smem& S, int k) {
             double pap = 0.0, z1 = 0.0, z2 = 0.0;
             for (int t = threadIdx.x; t < sc.rows; t += T) {
                 const int i = sc.row0 + t;
-                const int L = o.len[i];
-                int64_t at = sell_index(o.off[i >> 5], i & 31, 0);
-                double acc = 0.0;
-                for (int kk = 0; kk < L; kk++, at += kSellRows) acc = fma(o.val[at], B.p64[o.col[at]], acc);
+                const double acc = batch_row64(o, i, B.p64);
                 B.Ap64[i] = acc;
                 pap += B.p64[i] * acc;
             }
