@@ -272,15 +272,8 @@ __device__ __forceinline__ void product(const CgOperands& o, const LoopView& L, 
         for (int k = k0 - skip + warp + (warp < skip ? L.warps : 0); k < k1; k += L.warps) {
             const ChunkInfo c = L.info[k - table0];
             const T* p = part + c.first * 32 + lane;
-            T s = c.units > 0 ? p[0] : T(0);  // two chains of additions
-            if (c.units > 1) {
-                T q = p[32];
-                for (int u = 2; u < c.units; u++) {
-                    if (u & 1) q += p[u * 32];
-                    else s += p[u * 32];
-                }
-                s += q;
-            }
+            T s = c.units > 0 ? p[0] : T(0);  // in ascending columns, as the units are
+            for (int u = 1; u < c.units; u++) s += p[u * 32];
             const int row = c.chunk * kSellRows + lane;
             if (row >= L.lo && row < L.hi) f(k * kSellRows + lane, row, s);
         }
