@@ -423,6 +423,78 @@ __device__ __forceinline__ void for_near(const SceneConst& sc, const DeviceState
     }
 }
 
+// Neighbour walks of small scenes: kLanes lanes per particle.  A walk is a chain of 45 pairs
+// of 2,500 cycles each (FP64 operations answer after 64 cycles, square roots and quotients
+// after 400), and up to some 20,000 particles one lane each leaves most schedulers without a
+// warp or with one.  Eight lanes take eight pairs at once and park their terms in shared
+// memory; each accumulator is then one lane's, which adds its terms in list order, so every
+// sum is the one-lane walk's bit for bit (a pair without a term adds +0: sums_from_zero).
+constexpr int kLanes = 8;
+constexpr int kLaneGroups = 8;  // particles of a block
+constexpr int kLaneBlock = kLanes * kLaneGroups;
+
+template <int NA>
+struct LaneShared {
+    double term[kLaneGroups][kLanes][NA];
+    int near[kLaneGroups][8 * kLanes];
+};
+
+// f(j, term) for the candidates j of for_near in list order, eight at a time (j < 0: none):
+// called by all lanes of a warp together, it fills the lane's NA terms.  Returns, in lane
+// g < NA of the particle's lanes, the sum of terms g.  Every lane of the warp calls it.
+template <int NA, class F>
+__device__ __forceinline__ double near_by_lanes(const SceneConst& sc, const DeviceState& st, int i, bool active,
+                                                float out_thr, LaneShared<NA>& sh, F f) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kRounds = static_cast<int>(sizeof(sh.near[0]) / sizeof(int)) / kLanes;
+    const int lane = threadIdx.x & 31, g = lane & (kLanes - 1), first = lane & ~(kLanes - 1);
+    const int group = threadIdx.x / kLanes;
+    const int cnt = active ? st.nb_count[i] : 0;
+    float xi = 0.0f, zi = 0.0f;
+    if (active) {
+        xi = st.x32[i];
+        zi = st.z32[i];
+    }
+    const float si = fabsf(xi) + fabsf(zi);
+    double acc = 0.0;
+    for (int base = 0; __any_sync(kAll, base < cnt); base += kRounds * kLanes) {
+        int jj[kRounds];
+        float xj[kRounds], zj[kRounds];
+#pragma unroll
+        for (int s = 0; s < kRounds; s++) {
+            const int t = base + s * kLanes + g;
+            jj[s] = t < cnt ? st.nb[static_cast<int64_t>(t) * sc.n + i] : -1;
+        }
+#pragma unroll
+        for (int s = 0; s < kRounds; s++) {
+            xj[s] = jj[s] >= 0 ? st.x32[jj[s]] : 0.0f;
+            zj[s] = jj[s] >= 0 ? st.z32[jj[s]] : 0.0f;
+        }
+        int found = 0;
+#pragma unroll
+        for (int s = 0; s < kRounds; s++) {
+            const bool in = jj[s] >= 0 && !surely_out(xi, zi, si, xj[s], zj[s], out_thr);
+            const unsigned b = __ballot_sync(kAll, in) >> first & ((1u << kLanes) - 1u);
+            if (in) sh.near[group][found + __popc(b & ((1u << g) - 1u))] = jj[s];
+            found += __popc(b);
+        }
+        __syncwarp();
+        for (int k = 0; __any_sync(kAll, k < found); k += kLanes) {
+            double* term = sh.term[group][g];
+#pragma unroll
+            for (int a = 0; a < NA; a++) term[a] = 0.0;
+            f(k + g < found ? sh.near[group][k + g] : -1, term);
+            __syncwarp();
+            if (g < NA) {
+#pragma unroll
+                for (int q = 0; q < kLanes; q++) acc += sh.term[group][q][g];
+            }
+            __syncwarp();
+        }
+    }
+    return acc;
+}
+
 // for_near for three-dimensional scenes (surely_out3 on x32, y32, z32).
 template <class F>
 __device__ __forceinline__ void for_near3(const SceneConst& sc, const DeviceState& st, int i,

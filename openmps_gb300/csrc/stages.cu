@@ -348,6 +348,74 @@ __global__ void k_pre_pressure(SceneConst sc, DeviceState st) {
     add_gravity(sc, xi, zi, vx, vz, st.dux[i], st.duz[i]);
 }
 
+// k_pre_pressure with kLanes lanes per particle (near_by_lanes).
+template <bool kEcs>
+__global__ void __launch_bounds__(kLaneBlock) k_pre_pressure_lanes(SceneConst sc, DeviceState st) {
+    __shared__ LaneShared<4> sh;
+    if (step_failed(sc, st)) return;
+    const int i = static_cast<int>(blockIdx.x * kLaneGroups + threadIdx.x / kLanes);
+    const LapFactors lf = lap_factors(sc);
+    const bool spp = has_flag(sc.flags, MPS_FLAG_SPP);
+    const int first = threadIdx.x & 31 & ~(kLanes - 1);
+    const bool lead = (threadIdx.x & (kLanes - 1)) == 0;
+    const int t = i < sc.n ? st.type[i] : MPS_TYPE_DISABLED;
+    const bool active = t != MPS_TYPE_DUMMY && t != MPS_TYPE_DISABLED;
+    if (spp && lead && i < sc.n) st.n_wo_spp[i] = sc.n0;
+    const bool fluid = t == MPS_TYPE_FLUID;
+    const bool hs = kEcs && has_flag(sc.flags, MPS_FLAG_HS);
+    double xi = 0.0, zi = 0.0, ui = 0.0, wi = 0.0;
+    if (active) {
+        xi = st.x[i];
+        zi = st.z[i];
+        ui = st.u[i];
+        wi = st.w[i];
+    }
+    const float out_thr = fluid ? fmaxf(sc.f32_out_re, sc.f32_out_rl) : sc.f32_out_re;
+    const double acc = near_by_lanes<4>(sc, st, i, active, out_thr, sh, [&](int j, double* term) {
+        if (j < 0) return;
+        const double dx = st.x[j] - xi;
+        const double dz = st.z[j] - zi;
+        const double r2 = dist2(dx, dz);
+        const bool in_re = below(r2, sc.re2);
+        const bool in_rl = fluid && below(r2, sc.rl2);
+        if (!in_re && !in_rl) return;
+        const double r = dsqrt_rn(r2);
+        const double du = st.u[j] - ui;
+        const double dw = st.w[j] - wi;
+        if (in_re) {
+            term[0] = weight(r, sc.re);
+            if (hs) term[1] = ddiv_rn(dot2_term(dx, dz, du, dw), r * r * r);
+        }
+        if (in_rl && st.type[j] != MPS_TYPE_DUMMY) {
+            const double c = viscosity_coefficient(sc, lf, r);
+            term[2] = c * du;
+            term[3] = c * dw;
+        }
+    });
+    const double thisN = __shfl_sync(0xffffffffu, acc, first), hsum = __shfl_sync(0xffffffffu, acc, first + 1);
+    const double vx = __shfl_sync(0xffffffffu, acc, first + 2), vz = __shfl_sync(0xffffffffu, acc, first + 3);
+    if (!active || !lead) return;
+    double nd;
+    if (spp) {
+        st.n_wo_spp[i] = thisN;
+        nd = (thisN < sc.n0) ? sc.n0 : thisN;
+    } else {
+        nd = thisN;
+    }
+    st.nd[i] = nd;
+    if (kEcs) {
+        double speed;
+        if (has_flag(sc.flags, MPS_FLAG_HS)) {
+            speed = (spp && thisN < sc.n0) ? 0.0 : -sc.re * hsum;
+        } else {
+            speed = (nd - sc.n0) / st.step->dt;
+        }
+        const double error = (nd - sc.n0) / sc.n0;
+        st.ecs[i] = fabs(error) * speed + fabs(speed) * error;
+    }
+    if (fluid) add_gravity(sc, xi, zi, vx, vz, st.dux[i], st.duz[i]);
+}
+
 // ComputeExplicitForces, second loop (Computer.hpp:995-1020).
 __global__ void k_explicit_update(SceneConst sc, DeviceState st) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -569,6 +637,110 @@ __global__ void k_density_ppe(SceneConst sc, DeviceState st) {
     pr.diag(sc, st, a_ii);
 }
 
+// k_density_ppe with kLanes lanes per particle (near_by_lanes): a lane's place among the
+// row's entries and among those within r_e is the count of the lanes before it.
+__global__ void __launch_bounds__(kLaneBlock) k_density_ppe_lanes(SceneConst sc, DeviceState st) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ LaneShared<5> sh;
+    if (step_failed(sc, st)) return;
+    const int n = sc.n;
+    const int i = static_cast<int>(blockIdx.x * kLaneGroups + threadIdx.x / kLanes);
+    const LapFactors lf = lap_factors(sc);
+    const int g = threadIdx.x & (kLanes - 1), first = threadIdx.x & 31 & ~(kLanes - 1);
+    const unsigned before = (1u << g) - 1u;
+    const int t = i < n ? st.type[i] : MPS_TYPE_DISABLED;
+    const bool active = t != MPS_TYPE_DUMMY && t != MPS_TYPE_DISABLED;
+    const int row = i < n ? ppe_row(st, i) : 0;
+    if (i < n && g == 0) st.n_wo_spp[i] = sc.n0;
+    if (i < n && !active && g == 0) {
+        st.ppe_b[row] = 0;
+        st.ppe_x[row] = 0;
+        PpeRow(i, row).diag(sc, st, 1.0);
+    }
+    const bool hs = has_flag(sc.flags, MPS_FLAG_HS);
+    double xi = 0.0, zi = 0.0, ui = 0.0, wi = 0.0;
+    if (active) {
+        xi = st.x[i];
+        zi = st.z[i];
+        ui = st.u[i];
+        wi = st.w[i];
+    }
+    int m_re = 0;
+    PpeRow pr(i, row);
+    auto votes = [&](bool p) { return __ballot_sync(kAll, p) >> first & ((1u << kLanes) - 1u); };
+    const double acc = near_by_lanes<5>(sc, st, i, active, fmaxf(sc.f32_out_re, sc.f32_out_rl), sh, [&](int j, double* term) {
+        bool in_re = false, put = false;
+        int col = 0;
+        double w = 0.0, a_ij = 0.0;
+        if (j >= 0) {
+            const double dx = st.x[j] - xi;
+            const double dz = st.z[j] - zi;
+            const double r2 = dist2(dx, dz);
+            in_re = below(r2, sc.re2);
+            const bool in_rl = below(r2, sc.rl2);
+            if (in_re || in_rl) {
+                const double r = dsqrt_rn(r2);
+                w = in_re ? weight(r, sc.re) : 0.0;
+                term[0] = w;
+                if (in_re && hs)
+                    term[1] = ddiv_rn(dot2_term(dx, dz, st.u[j] - ui, st.w[j] - wi), r * r * r);
+                if (in_rl) {
+                    if (st.type[j] != MPS_TYPE_DUMMY) {
+                        a_ij = ppe_coefficient(sc, lf, r);
+                        put = true;
+                        col = ppe_row(st, j);
+                        term[2] = -a_ij;
+                    }
+                    const double wg = (in_re && sc.re_lap == sc.re) ? w : weight(r, sc.re_lap);
+                    term[3] = wg * dx;
+                    term[4] = wg * dz;
+                }
+            }
+        }
+        const unsigned re = votes(in_re), puts = votes(put), low = votes(put && col < row);
+        const int mine = m_re + __popc(re & before);
+        if (in_re && mine < kReCache) st.w_re[static_cast<int64_t>(mine) * n + i] = w;
+        m_re += __popc(re);
+        // the column before this lane's, and the last one
+        const int left = 31 - __clz(puts & before), last = 31 - __clz(puts);
+        const int left_col = __shfl_sync(kAll, col, first + max(left, 0));
+        const int last_col = __shfl_sync(kAll, col, first + max(last, 0));
+        if (put) {
+            PpeRow lane(i, row);
+            lane.m = pr.m + __popc(puts & before);
+            lane.prev = left >= 0 ? left_col : pr.prev;
+            lane.put(sc, st, col, a_ij);
+        }
+        pr.m += __popc(puts);
+        pr.below += __popc(low);
+        if (last >= 0) pr.prev = last_col;
+    });
+    const double thisN = __shfl_sync(kAll, acc, first), hsum = __shfl_sync(kAll, acc, first + 1);
+    double a_ii = __shfl_sync(kAll, acc, first + 2);
+    const double gx = __shfl_sync(kAll, acc, first + 3), gz = __shfl_sync(kAll, acc, first + 4);
+    if (!active || g != 0) return;
+    st.n_wo_spp[i] = thisN;
+    const double nd = (thisN < sc.n0) ? sc.n0 : thisN;
+    st.nd[i] = nd;
+    const double dt = st.step->dt;
+    const double speed = hs ? ((thisN < sc.n0) ? 0.0 : -sc.re * hsum) : (nd - sc.n0) / dt;
+    if (has_flag(sc.flags, MPS_FLAG_ECS)) {
+        const double e = st.ecs[i];
+        st.ppe_b[row] = -sc.rho / (sc.n0 * dt) * (speed + e);
+    } else {
+        st.ppe_b[row] = -sc.rho / (sc.n0 * dt) * speed;
+    }
+    st.ppe_x[row] = st.p[i];
+    st.spp_g[i] = gx;
+    st.spp_g[n + i] = gz;
+    double xs, zs;
+    if (spp_particle(sc, st, i, sc.re_lap, gx, gz, xs, zs)) {
+        const double ddx = xi - xs, ddz = zi - zs;
+        a_ii += -ppe_coefficient(sc, lf, dsqrt_rn(dot2(ddx, ddz, ddx, ddz)));
+    }
+    pr.diag(sc, st, a_ii);
+}
+
 // Chunk sizes of the SELL-32 layout: one warp per chunk of 32 rows.
 __global__ void k_ppe_chunks(SceneConst sc, DeviceState st) {
     const int c = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -686,6 +858,70 @@ __global__ void k_pressure_gradient(SceneConst sc, DeviceState st) {
         sx += c * dx;
         sz += c * dz;
     }
+    st.dux[i] = factor * sx;
+    st.duz[i] = factor * sz;
+}
+
+// k_pressure_gradient with kLanes lanes per particle (near_by_lanes).
+template <int kCache>
+__global__ void __launch_bounds__(kLaneBlock) k_pressure_gradient_lanes(SceneConst sc, DeviceState st) {
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ LaneShared<4> sh;
+    if (solve_failed(sc, st)) return;
+    const int i = static_cast<int>(blockIdx.x * kLaneGroups + threadIdx.x / kLanes);
+    const int g = threadIdx.x & (kLanes - 1), first = threadIdx.x & 31 & ~(kLanes - 1);
+    const bool active = i < sc.n && st.type[i] == MPS_TYPE_FLUID;
+    const bool spp = has_flag(sc.flags, MPS_FLAG_SPP);
+    double xi = 0.0, zi = 0.0, pi = 0.0;
+    if (active) {
+        xi = st.x[i];
+        zi = st.z[i];
+        pi = st.p[i];
+    }
+    int m_re = 0;
+    const double acc = near_by_lanes<4>(sc, st, i, active, sc.f32_out_re, sh, [&](int j, double* term) {
+        double dx = 0.0, dz = 0.0, r2 = 0.0;
+        bool in_re = false;
+        if (j >= 0) {
+            dx = st.x[j] - xi;
+            dz = st.z[j] - zi;
+            r2 = dist2(dx, dz);
+            in_re = below(r2, sc.re2);
+        }
+        const unsigned re = __ballot_sync(kAll, in_re) >> first & ((1u << kLanes) - 1u);
+        const int mine = m_re + __popc(re & ((1u << g) - 1u));
+        m_re += __popc(re);
+        if (!in_re) return;
+        const double wg = (kCache >= 1 && mine < kReCache) ? st.w_re[static_cast<int64_t>(mine) * sc.n + i]
+                                                          : weight(dsqrt_rn(r2), sc.re);
+        if (st.type[j] != MPS_TYPE_DUMMY) {
+            const double c = ddiv_rn(st.p[j] + pi, r2) * wg;
+            term[0] = c * dx;
+            term[1] = c * dz;
+        }
+        if (kCache < 2 && spp) {
+            term[2] = wg * dx;
+            term[3] = wg * dz;
+        }
+    });
+    double sx = __shfl_sync(kAll, acc, first), sz = __shfl_sync(kAll, acc, first + 1);
+    double gx = __shfl_sync(kAll, acc, first + 2), gz = __shfl_sync(kAll, acc, first + 3);
+    if (!active || g != 0) return;
+    if (kCache == 2 && spp) {
+        gx = st.spp_g[i];
+        gz = st.spp_g[sc.n + i];
+    }
+    double xs, zs;
+    if (spp && spp_particle(sc, st, i, sc.re, gx, gz, xs, zs)) {
+        const double dx = xs - xi;
+        const double dz = zs - zi;
+        const double r2 = dist2(dx, dz);
+        const double c = ddiv_rn(0.0 + pi, r2) * weight(dsqrt_rn(r2), sc.re);
+        sx += c * dx;
+        sz += c * dz;
+    }
+    const double dt = st.step->dt;
+    const double factor = -dt / sc.rho * 2.0 / sc.n0;
     st.dux[i] = factor * sx;
     st.duz[i] = factor * sz;
 }
@@ -896,7 +1132,22 @@ void launch_density_variation(const SceneConst& sc, const DeviceState& st, doubl
     k_density_variation<<<grid_for(sc.n), kBlock, 0, s>>>(sc, st, out);
 }
 
+// Whether the walks take kLanes lanes per particle (near_by_lanes).  us of density + ECS +
+// explicit, of density + assembly and of the gradient, one lane against eight: 1,850
+// particles 113 / 27, 156 / 37, 72 / 27; 16,850 122 / 62, 168 / 86, 78 / 53; 25,050 131 / 91,
+// 172 / 111, 82 / 70; 42,226 146 / 140, 190 / 172, 92 / 110; 90,050 242 / 287, 279 / 354,
+// 150 / 219 (an accumulator's addition takes the FP64 pipe 64 cycles for 4 particles there,
+// for 32 with one lane each).
+bool by_lanes(const SceneConst& sc) { return sc.n <= 32768; }
+
 void launch_pre_pressure(const SceneConst& sc, const DeviceState& st, cudaStream_t s) {
+    if (by_lanes(sc)) {
+        if ((sc.flags & MPS_FLAG_ECS) != 0u)
+            k_pre_pressure_lanes<true><<<grid_for(sc.n, kLaneGroups), kLaneBlock, 0, s>>>(sc, st);
+        else
+            k_pre_pressure_lanes<false><<<grid_for(sc.n, kLaneGroups), kLaneBlock, 0, s>>>(sc, st);
+        return;
+    }
     if ((sc.flags & MPS_FLAG_ECS) != 0u)
         k_pre_pressure<true><<<grid_for(sc.n, kWalkBlock), kWalkBlock, 0, s>>>(sc, st);
     else
@@ -944,7 +1195,10 @@ bool density_ppe_fusable(const SceneConst& sc) {
 }
 
 void launch_density_set_ppe(const SceneConst& sc, const DeviceState& st, bool want_fp32, cudaStream_t s) {
-    k_density_ppe<<<grid_for(sc.n, kWalkBlock), kWalkBlock, 0, s>>>(sc, assembly_state(st, want_fp32));
+    if (by_lanes(sc))
+        k_density_ppe_lanes<<<grid_for(sc.n, kLaneGroups), kLaneBlock, 0, s>>>(sc, assembly_state(st, want_fp32));
+    else
+        k_density_ppe<<<grid_for(sc.n, kWalkBlock), kWalkBlock, 0, s>>>(sc, assembly_state(st, want_fp32));
     launch_ppe_layout(sc, st, want_fp32, s);
 }
 
@@ -964,6 +1218,8 @@ void launch_density_explicit_pressure(const SceneConst& sc, const DeviceState& s
 void launch_pressure_gradient(const SceneConst& sc, const DeviceState& st, cudaStream_t s) {
     if (sc.flags & MPS_FLAG_GC)
         k_pressure_gradient_gc<0><<<grid_for(sc.n, kWalkBlock), kWalkBlock, 0, s>>>(sc, st);
+    else if (by_lanes(sc))
+        k_pressure_gradient_lanes<0><<<grid_for(sc.n, kLaneGroups), kLaneBlock, 0, s>>>(sc, st);
     else
         k_pressure_gradient<0><<<grid_for(sc.n, kWalkBlock), kWalkBlock, 0, s>>>(sc, st);
     k_apply_du<<<grid_for(sc.n), kBlock, 0, s>>>(sc, st);
@@ -978,6 +1234,12 @@ void launch_pressure_gradient_cached(const SceneConst& sc, const DeviceState& st
             k_pressure_gradient_gc<2><<<g, kWalkBlock, 0, s>>>(sc, st);
         else
             k_pressure_gradient_gc<1><<<g, kWalkBlock, 0, s>>>(sc, st);
+    } else if (by_lanes(sc)) {
+        const unsigned gl = grid_for(sc.n, kLaneGroups);
+        if (spp_sums)
+            k_pressure_gradient_lanes<2><<<gl, kLaneBlock, 0, s>>>(sc, st);
+        else
+            k_pressure_gradient_lanes<1><<<gl, kLaneBlock, 0, s>>>(sc, st);
     } else if (spp_sums) {
         k_pressure_gradient<2><<<g, kWalkBlock, 0, s>>>(sc, st);
     } else {
