@@ -59,8 +59,13 @@ constexpr int kRowBytes = 5 * 4, kWindowBytes = 4 + 4 + 2, kCellBytes = 4 + 4 + 
 struct BottomLevel {
     int nx, nz, cells;
     int k, dinv, r, e, x;  // float offsets
-    unsigned by_nz;        // quotients by nz: __umulhi(c, by_nz) for c nz < 2^32
+    unsigned by_nz;        // of column_of
 };
+
+// c / nz for c nz < 2^32 (2^32 / 1 has no 32-bit multiplier)
+__device__ __forceinline__ int column_of(const BottomLevel& B, int c) {
+    return B.nz == 1 ? c : static_cast<int>(__umulhi(static_cast<unsigned>(c), B.by_nz));
+}
 
 __host__ __device__ inline int bottom_level_floats(const MgLevel& L, bool last) {
     const int64_t c = mg_round4(L.cells);
@@ -336,7 +341,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
                 const float r = src[c];
                 bot[B.r + c] = r;
                 if (plan.bottom < mg.levels) {
-                    const int cx = static_cast<int>(__umulhi(static_cast<unsigned>(c), B.by_nz));
+                    const int cx = column_of(B, c);
                     bot[B.x + (cx + 1) * (B.nz + 2) + c - cx * B.nz + 1] = bot[B.dinv + c] * r;
                 }
             }
@@ -359,7 +364,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
             const BottomLevel B = bl[l], C = bl[l + 1];
             for (int I = t >> 2; I - (t >> 2) < C.cells; I += nt >> 2) {
                 const int cell = min(I, C.cells - 1);
-                const int X = static_cast<int>(__umulhi(static_cast<unsigned>(cell), C.by_nz)), Z = cell - X * C.nz;
+                const int X = column_of(C, cell), Z = cell - X * C.nz;
                 const int cx = 2 * X + ((t >> 1) & 1), cz = 2 * Z + (t & 1);
                 float v = cx < B.nx && cz < B.nz ? residual(B, cx, cz) : 0.0f;
                 v += __shfl_xor_sync(0xffffffffu, v, 1);
@@ -387,12 +392,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
         for (int l = mg.levels - 1; l >= plan.bottom; l--) {
             const BottomLevel B = bl[l], C = bl[l + 1];
             for (int c = t; c < B.cells; c += nt) {  // x += w e of the parent
-                const int cx = static_cast<int>(__umulhi(static_cast<unsigned>(c), B.by_nz)), cz = c - cx * B.nz;
+                const int cx = column_of(B, c), cz = c - cx * B.nz;
                 bot[B.x + (cx + 1) * (B.nz + 2) + cz + 1] += kMgCoarseWeight * bot[C.e + (cx >> 1) * C.nz + (cz >> 1)];
             }
             __syncthreads();
             for (int c = t; c < B.cells; c += nt) {  // and one Jacobi step
-                const int cx = static_cast<int>(__umulhi(static_cast<unsigned>(c), B.by_nz)), cz = c - cx * B.nz;
+                const int cx = column_of(B, c), cz = c - cx * B.nz;
                 bot[B.e + c] = bot[B.x + (cx + 1) * (B.nz + 2) + cz + 1] + bot[B.dinv + c] * residual(B, cx, cz);
             }
             __syncthreads();

@@ -2,7 +2,7 @@
 
 Scenes around the largest system one cluster takes (2,560 rows), with hierarchies whose
 single-block levels start at level 1, 2 and deeper, columns of cells much taller and much
-shorter than usual, and cells so full that a block's window overflows (u goes through
+shorter than usual (coarse levels one cell high), and cells so full that a block's window overflows (u goes through
 global memory).
 
 Tolerance: a column of N particles under a free surface has a condition number of about
@@ -24,6 +24,7 @@ CASES = {
     "few_rows": (2e-2, 0.1, 0.06, 0.2, 0.2, 2.1),
     "grid": (4e-3, 0.2, 0.4, 0.8, 0.6, 2.1),
     "flat": (5e-3, 2.0, 0.03, 6.0, 0.06, 2.1),
+    "film": (5e-3, 1.0, 0.015, 14.0, 0.02, 2.1),
     "tall": (5e-3, 0.06, 1.0, 0.1, 1.2, 2.1),
     "deep_bottom": (2e-3, 0.2, 0.2, 2.0, 0.8, 2.1),
     "full_cells": (2e-3, 0.1, 0.4, 0.12, 0.4, 6.0),
