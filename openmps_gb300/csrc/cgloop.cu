@@ -372,6 +372,8 @@ LoopPlan loop_plan(int nchunks, bool cluster, int keep_row_bytes) {
     p.blocks = cluster ? g_loop_cluster : g_loop_sms;
     if (!cluster && p.blocks > nchunks) p.blocks = nchunks;
     const int per = (nchunks + p.blocks - 1) / p.blocks;
+    // two or three times the average share (a block of thin chunks alone can own five times
+    // it, and then works in tiles)
     p.tables = kTileChunks;
     if (table_bytes(3 * per + 2) <= g_loop_smem / 2)
         p.tables = 3 * per + 2;

@@ -655,6 +655,9 @@ void launch_density3(const SceneConst& sc, const DeviceState& st, cudaStream_t s
 void launch_error_correction3(const SceneConst& sc, const DeviceState& st, cudaStream_t s);
 void launch_density_variation3(const SceneConst& sc, const DeviceState& st, double* out, cudaStream_t s);
 void launch_explicit3(const SceneConst& sc, const DeviceState& st, cudaStream_t s);
+void launch_pre_pressure3(const SceneConst& sc, const DeviceState& st, cudaStream_t s);
+void launch_explicit_update3(const SceneConst& sc, const DeviceState& st, cudaStream_t s);
+void launch_density_set_ppe3(const SceneConst& sc, const DeviceState& st, bool want_fp32, cudaStream_t s);
 void launch_save_x3(const SceneConst& sc, const DeviceState& st, cudaStream_t s);
 void launch_set_ppe3(const SceneConst& sc, const DeviceState& st, bool want_fp32, cudaStream_t s);
 void launch_pressure_gradient3(const SceneConst& sc, const DeviceState& st, cudaStream_t s);

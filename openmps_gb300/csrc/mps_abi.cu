@@ -831,28 +831,31 @@ void forward3(mps_handle* h, double dt) {
         launched(h, kLaunchesCfl);
     }
     do_search(h);
+    // the walks share as in two dimensions, and so do the stage times
     stage_mark(h, kDensity);
-    launch_density3(sc, h->st, s);
-    launched(h, kLaunchesDensity);
+    launch_pre_pressure3(sc, h->st, s);
+    launched(h, kLaunchesPrePressure);
     stage_mark(h, kEcs);
-    if (flags & MPS_FLAG_ECS) {
-        launch_error_correction3(sc, h->st, s);
-        launched(h, kLaunchesEcs);
-    }
     stage_mark(h, kExplicit);
-    launch_explicit3(sc, h->st, s);
-    launched(h, kLaunchesExplicit);
+    launch_explicit_update3(sc, h->st, s);
+    launched(h, kLaunchesExplicitUpdate);
     stage_mark(h, kDensity2);
-    launch_density3(sc, h->st, s);
-    launched(h, kLaunchesDensity);
+    const bool implicit = (flags & MPS_FLAG_PRESSURE_EXPLICIT) == 0u;
+    const bool fused = density_ppe_fusable(sc);
+    if (!fused) {
+        launch_density3(sc, h->st, s);
+        launched(h, kLaunchesDensity);
+    }
     if (flags & MPS_FLAG_DS) {
         launch_save_x3(sc, h->st, s);
         launched(h, kLaunchesSaveX);
     }
-    const bool implicit = (flags & MPS_FLAG_PRESSURE_EXPLICIT) == 0u;
     stage_mark(h, kPpe);
     if (implicit) {
-        launch_set_ppe3(sc, h->st, wants_fp32(h), s);
+        if (fused)
+            launch_density_set_ppe3(sc, h->st, wants_fp32(h), s);
+        else
+            launch_set_ppe3(sc, h->st, wants_fp32(h), s);
         h->ppe_fp32 = wants_fp32(h);
         launched(h, set_ppe_launches(h->st));
         after_launch("stages");
