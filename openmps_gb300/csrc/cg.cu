@@ -435,6 +435,8 @@ __device__ __forceinline__ void pmx_finish(CgScalars* S, int mode, const double*
         stalled = !(std::isfinite(alpha) && std::isfinite(beta) && alpha != 0.0);
         S->alpha = alpha;
         S->beta = beta;
+        S->alpha32 = __double2float_rn(alpha);
+        S->beta32 = __double2float_rn(beta);
         S->rr = gam;
         S->pAp = del;
     }
@@ -476,12 +478,12 @@ __global__ void __launch_bounds__(kBlock, 5) k_pmx_spmv(CgOperands o, int mode,
     double vg = 0.0, vd = 0.0, vr = 0.0;
     auto row_done = [&](int i, float wi, float rf) {
         if (i < o.n) {
-            const double ri = static_cast<double>(rf);
-            const double ui = static_cast<double>(u[i]);
+            const double ri = widen(rf);
+            const double ui = widen(u[i]);
             o.w32[i] = wi;
             if (mode == 2) o.d32[i] = 0.0f;
             vg += ri * ui;
-            vd += static_cast<double>(wi) * ui;
+            vd += widen(wi) * ui;
             vr += ri * ri;
         }
     };

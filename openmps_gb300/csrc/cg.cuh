@@ -43,6 +43,7 @@ struct CgScalars {
     int32_t fb_iter;      // iterations of that fallback
     int32_t iter_upd;     // MIXED: iteration of the last reliable update
     double prev_true_rr;  // true r.r at the previous reliable update
+    float alpha32, beta32;  // rounded once (a conversion takes the FP64 pipe 64 cycles a warp)
 };
 
 struct CgOperands {

@@ -300,8 +300,7 @@ __global__ void __launch_bounds__(kBlock) k_mg_axpy_restrict(CgOperands o, MgLev
     }
     pdl_begin();  // the step sizes and the vectors come from the SpMV just before
     if (pcg_skip(o.S, 1)) return;
-    const float alpha = __double2float_rn(o.S->alpha);
-    const float beta = __double2float_rn(o.S->beta);
+    const float alpha = o.S->alpha32, beta = o.S->beta32;
     for (int base = base0; base < nact; base += 2 * nwarps) {
         const int a = base + half;
         float sum = 0.0f;
