@@ -791,11 +791,24 @@ __global__ void k_ppe_sort(SceneConst sc, DeviceState st, int want_fp32) {
         put(len - 1, below_diag);
         return;
     }
-    for (int e = 0; e < len; e++) {
-        const int ce = st.ppe_col_tmp[ell(e, n, i)];
-        int rank = 0;
-        for (int f = 0; f < len; f++) rank += (st.ppe_col_tmp[ell(f, n, i)] < ce) ? 1 : 0;
-        put(e, rank);
+    // eight entries' ranks from one pass over the columns (256 scenes, 53 M entries: 985 us
+    // against 1,090 with one entry a pass; what is left is put's stores, scattered by rank)
+    constexpr int kRanks = 8;
+    for (int e0 = 0; e0 < len; e0 += kRanks) {
+        int ce[kRanks], rank[kRanks];
+#pragma unroll
+        for (int u = 0; u < kRanks; u++) {
+            ce[u] = e0 + u < len ? st.ppe_col_tmp[ell(e0 + u, n, i)] : 0;
+            rank[u] = 0;
+        }
+        for (int f = 0; f < len; f++) {
+            const int cf = st.ppe_col_tmp[ell(f, n, i)];
+#pragma unroll
+            for (int u = 0; u < kRanks; u++) rank[u] += cf < ce[u] ? 1 : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kRanks; u++)
+            if (e0 + u < len) put(e0 + u, rank[u]);
     }
 }
 
