@@ -201,13 +201,15 @@ __device__ __forceinline__ bool aborted_before_solve(const CgOperands& o,
     return false;
 }
 
-// The width of chunk c for the single-launch loops, or 0 when they leave it out: every row
-// is an identity row (its diagonal alone) with a zero residual, so its x stays.  Warp per
-// chunk, lane = row i of length L at `at`, residual ri.
+// The width of chunk c for the single-launch loops (1 when none of its rows has an entry), or
+// 0 when they leave it out: every row has a zero residual and is an identity row (its
+// diagonal alone) or empty, so its x stays.  An empty row with a residual stays in: the
+// residual counts in r.r, so such a system never converges.  Warp per chunk, lane = row i of
+// length L at `at`, residual ri (0 past the last row).
 __device__ __forceinline__ void store_loop_width(const CgOperands& o, int c, int i, int L, int64_t at, double ri) {
-    const bool idle = L == 0 || (L == 1 && o.col[at] == i && ri == 0.0);
+    const bool idle = ri == 0.0 && (L == 0 || (L == 1 && o.col[at] == i));
     const bool out = __all_sync(kFull, idle);
-    if ((threadIdx.x & 31) == 0 && o.loop_w) o.loop_w[c] = out ? 0 : o.chunk[c] / kSellRows;
+    if ((threadIdx.x & 31) == 0 && o.loop_w) o.loop_w[c] = out ? 0 : max(1, o.chunk[c] / kSellRows);
 }
 
 // Entries of chunk c past row i's length L: {i, 0}, so that the loops add all entries of a

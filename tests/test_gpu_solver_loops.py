@@ -139,3 +139,37 @@ def test_noalloc_sizes(gpu_lib, name):
     assert rel.value <= 1.01e-12
     assert err <= TOL
     assert np.array_equal(got[0], got[1])
+
+
+# empty rows: an aligned chunk of them, and one at the end of a chunk of padding rows
+EMPTY = {"last_row": (33, np.arange(32, 33)), "middle_chunk": (96, np.arange(32, 64)),
+         "grid": (80 * 32 + 65, np.arange(3 * 32, 5 * 32))}
+
+
+@pytest.mark.parametrize("solver", ["cg64", "mixed"])
+@pytest.mark.parametrize("name", list(EMPTY))
+def test_empty_rows(gpu_lib, name, solver):
+    # 0 = b has no solution: the rows' residual stays in r.r whatever the rest does.  With
+    # b = 0 there the system is solved, and x keeps its start in those rows.
+    from openmps_gb300.computer import Computer, ComputerError
+
+    n, empty = EMPTY[name]
+    ptr, col, val, b, xs, x0 = _system(n, (1, 7), seed=n)
+    gone = np.zeros(n, bool)
+    gone[empty] = True
+    row = np.repeat(np.arange(n), np.diff(ptr))
+    keep = ~gone[row] & ~gone[col]
+    ptr = np.concatenate([[0], np.cumsum(np.bincount(row[keep], minlength=n))]).astype(np.int64)
+    col, val = col[keep], val[keep]
+    b = np.bincount(row[keep], weights=val * xs[col], minlength=n)
+    c = Computer(abi.make_params())
+    which = abi.SOLVER_CG64 if solver == "cg64" else abi.SOLVER_MIXED
+    x, _, rel = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    assert rel <= 1.01e-12
+    assert np.array_equal(x[empty], x0[empty])
+    assert np.linalg.norm((x - xs)[~gone]) <= TOL * np.linalg.norm(xs)
+    for size in (1e-3, 1.0):
+        b[empty] = size
+        with pytest.raises(ComputerError) as e:
+            c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, max_iters=200, solver=which)
+        assert e.value.code == abi.MPS_ERR_CG_NOT_CONVERGED
