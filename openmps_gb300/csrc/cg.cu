@@ -1530,7 +1530,9 @@ cudaError_t CgGraph::build_persistent(int solver, const CgOperands& ops, cudaStr
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         GridSync g{ps.count, ps.gen, ps.err, ps.limits};
-        cudaLaunchKernelEx(&cfg, k_pcg_persistent, ops, *mg, g);
+        CgOperands own = ops;
+        own.partials = ps.partials;
+        cudaLaunchKernelEx(&cfg, k_pcg_persistent, own, *mg, g);
     }
     const cudaError_t fe = fallback_kernels(ops, *fb, 0, s);  // the persistent loop records no true residual
     e = cudaStreamEndCapture(s, &captured);

@@ -217,7 +217,9 @@ constexpr long long kDefaultMmaClocks = 2000000000LL;      // about one second
 // kernel waits this long again for their completion before it frees TMEM.
 constexpr long long kMmaDrainClocks = 2000000000LL;
 
-// Device words of the persistent solve's grid barrier, and its grid size.
+// Device words of the persistent solve's grid barrier, its grid size and partial sums.  Its
+// grid is as large as the device holds whatever the rows, so its partial sums are its own
+// (CgOperands::partials is sized for the grids of the rows).
 constexpr int kPersistentCounters = 513;  // barrier group counters + the top one
 
 struct PersistentSync {
@@ -225,6 +227,7 @@ struct PersistentSync {
     unsigned* gen;
     int32_t* err;     // set when a barrier wait runs out
     int blocks;
+    double* partials;  // 3 x blocks
     const WaitLimits* limits;  // null: the defaults
 };
 

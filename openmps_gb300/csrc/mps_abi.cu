@@ -506,6 +506,8 @@ void allocate(mps_handle* h, int64_t n, int64_t keep) {
     h->psync.gen = dalloc<unsigned>(h, 1);
     h->psync.err = dalloc<int32_t>(h, 1);
     h->psync.limits = h->d_limits;
+    h->psync.blocks = persistent_blocks();
+    h->psync.partials = dalloc<double>(h, 3 * static_cast<int64_t>(h->psync.blocks));
     cudaStream_t s = h->stream;
     // zero everything persistent, then carry the old contents over
     check(cudaMemsetAsync(st.type, 0, sizeof(int32_t) * n, s), "memset");
@@ -789,11 +791,9 @@ void do_solve(mps_handle* h) {
             h->cg.persistent() != want_persistent) {
             bool built = false;
             if (want_persistent) {
-                PersistentSync ps = h->psync;
-                ps.blocks = persistent_blocks();
-                built = ps.blocks > 0 &&
-                        h->cg.build_persistent(solver, cg_operands(h), s, &mg, &fb, learned ? &run : nullptr, ps) ==
-                            cudaSuccess;
+                built = h->psync.blocks > 0 &&
+                        h->cg.build_persistent(solver, cg_operands(h), s, &mg, &fb, learned ? &run : nullptr,
+                                               h->psync) == cudaSuccess;
                 if (!built) {
                     // no cooperative launch in a graph on this device: per-phase kernels
                     cudaGetLastError();

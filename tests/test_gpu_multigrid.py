@@ -83,6 +83,37 @@ def test_persistent_kernel_matches_per_phase_kernels(gpu_lib, maker):
     assert abs(sa["cg_iterations"] - sb["cg_iterations"]) <= 2
 
 
+@pytest.mark.parametrize("l0", [2e-2, 1e-2, 5e-3])
+def test_persistent_kernel_keeps_to_its_buffers(gpu_lib, l0):
+    # the persistent grid is as large as the device holds, however few the rows: its steps
+    # leave what was allocated around its handle alone, so that handles created before and
+    # after it step as they do by themselves
+    s = scenes.dam_break(l0, 0.2, 0.4, 0.8, 0.6)
+    dt = 0.01 * l0
+
+    def handle(launch):
+        c = Computer(s.params(eps=1e-10, solver=abi.SOLVER_MIXED_MG, criterion=abi.CRIT_RHS, cg_launch=launch))
+        c.add_scene(s)
+        return c
+
+    alone = handle(abi.CG_LAUNCH_GRAPH)
+    for _ in range(4):
+        alone.forward_time(dt)
+    want = alone.particles()
+    group = [handle(k) for k in (abi.CG_LAUNCH_GRAPH, abi.CG_LAUNCH_PERSISTENT, abi.CG_LAUNCH_GRAPH,
+                                 abi.CG_LAUNCH_PERSISTENT, abi.CG_LAUNCH_GRAPH)]
+    for _ in range(4):
+        for c in group:
+            c.forward_time(dt)
+            assert c.stats()["fallback"] == 0 and c.stats()["cg_true_relres"] <= 1e-10
+    for c in group[::2]:
+        got = c.particles()
+        for k in ("x", "z", "u", "w", "p"):
+            np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+    for k in ("x", "z"):
+        np.testing.assert_array_equal(group[1].particles()[k], group[3].particles()[k], err_msg=k)
+
+
 def test_deterministic(gpu_lib):
     s = stock_tank()
     ps = []
