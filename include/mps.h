@@ -250,12 +250,15 @@ int mps_set_solver(mps_handle* h, int32_t solver, int32_t criterion, double eps)
 int mps_set_stage_timing(mps_handle* h, int32_t enable);
 /* Bounds of the handle's device-side waits, in SM clock cycles (negative: the default).
  * No counterpart in the reference, which has no device waits.  barrier_clocks bounds
- * each grid-barrier wait of the persistent preconditioned solve (MPS_CG_LAUNCH_PERSISTENT;
- * default 4e9, about two seconds); mma_clocks bounds each tensor-core completion wait of
- * the learned solve's network inference (default 2e9).  A wait that runs out sets an
- * error word and lets its kernel return: the step still completes (the network's
- * output is not used, or the FP64 CG finishes the solve), and mps_forward_time returns
- * MPS_ERR_TIMEOUT.  The handle stays usable.  0 makes every such wait give up at its
+ * each grid-wide exchange of the solvers' single-launch loops and each grid-barrier wait
+ * of the persistent preconditioned solve (MPS_CG_LAUNCH_PERSISTENT; default 4e9, about
+ * two seconds); small systems iterate in one cluster, whose hardware barrier is not such a
+ * wait.  mma_clocks bounds each tensor-core completion wait of the learned solve's
+ * network inference (default 2e9).  A wait that runs out sets an error word and lets its
+ * kernel return: the step still completes (the network's output is not used, or the FP64
+ * CG finishes a mixed-precision solve, under the default bounds), and mps_forward_time
+ * returns MPS_ERR_TIMEOUT.  MPS_SOLVER_CG64 has nothing to finish it: its step ends at
+ * the solve, like one that did not converge.  The handle stays usable.  0 makes every such wait give up at its
  * first check, which tests use to exercise this path. */
 int mps_set_wait_limits(mps_handle* h, int64_t barrier_clocks, int64_t mma_clocks);
 

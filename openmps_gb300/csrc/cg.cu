@@ -182,6 +182,7 @@ __device__ void init_scalars(CgScalars* S, double rr, double bb, cudaGraphCondit
     S->updates = 0;
     S->aborted = 0;
     S->stalled = 0;
+    S->timed_out = 0;
     S->prev_true_rr = rr;
     S->iter_upd = 0;
     if (use_cond) cudaGraphSetConditional(h, (!conv && S->max_iter > 0) ? 1u : 0u);
@@ -229,10 +230,11 @@ __device__ __forceinline__ void pad_row(const CgOperands& o, int c, int i, int L
 // fallback after a preconditioned solve) nothing runs unless that solve failed.
 __global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, const CgScalars* gate) {
     __shared__ BlockTicket tk;
-    if (gate && (gate->converged || gate->aborted)) {
+    if (gate && (gate->aborted || (gate->converged && !gate->timed_out))) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             o.S->converged = gate->converged;
             o.S->aborted = gate->aborted;
+            o.S->timed_out = 0;
             o.S->iter = 0;
         }
         return;
@@ -388,7 +390,7 @@ __device__ __forceinline__ void true_residual_done(CgScalars* S, double rr, cuda
 
 // After the loop: the solution into x (fold a pending correction, leave the x2 buffer).
 __global__ void __launch_bounds__(kBlock) k_mx_finish(CgOperands o) {
-    if (o.S->aborted) return;
+    if (o.S->aborted || o.S->timed_out) return;  // timed out: x stays an iterate, the FP64 CG starts from it
     const bool odd = (o.S->updates & 1) != 0;
     const bool folded = o.S->do_update != 0;
     const double* xc = odd ? o.x2 : o.x;
@@ -787,7 +789,7 @@ void launch_pmx_spmv(const CgOperands& o, int mode, cudaGraphConditionalHandle h
 // After the fallback: report it in the primary scalars.
 __global__ void k_fb_merge(CgScalars* S, const CgScalars* F) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (S->converged || S->aborted) return;
+    if (S->aborted || (S->converged && !S->timed_out)) return;
     S->fallback = 1;
     S->fb_iter = F->iter;
     S->converged = F->converged;
@@ -805,6 +807,7 @@ __global__ void k_cg_configure(CgScalars* S, double eps, int criterion, int max_
         S->converged = 0;
         S->iter = 0;
         S->aborted = 0;
+        S->timed_out = 0;
         S->do_update = 0;
         S->updates = 0;
         S->stalled = 0;

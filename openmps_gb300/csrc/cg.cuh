@@ -15,6 +15,8 @@ __device__ __forceinline__ uint2 ld_sell_pair(const uint2* p) {
     return e;
 }
 
+struct WaitLimits;
+
 // Scalars of one solve, in device memory (read back once per step).
 struct CgScalars {
     double rr;        // r.r of the current direction update
@@ -44,6 +46,7 @@ struct CgScalars {
     int32_t iter_upd;     // MIXED: iteration of the last reliable update
     double prev_true_rr;  // true r.r at the previous reliable update
     float alpha32, beta32;  // rounded once (a conversion takes the FP64 pipe 64 cycles a warp)
+    int32_t timed_out;  // a wait of the single-launch loop ran out; last: see store_scalars
 };
 
 struct CgOperands {
@@ -73,6 +76,7 @@ struct CgOperands {
     int32_t* loop_w;    // per chunk: its width, 0 when the loops leave it out (written by init)
     CgScalars* S;
     const DevStatus* status;  // step status (may be null): a failed search aborts the solve
+    const WaitLimits* limits;  // bounds of the loops' waits (null: the defaults)
 };
 
 // Row i (lane of a chunk at `at`) times v in FP64, ascending columns.  The FP64 matrix
@@ -208,7 +212,7 @@ cudaError_t cg_loop_prepare_device();
 // cycles have passed since it began (0: at its first check), sets an error word and
 // lets its kernel return; the host turns the word into MPS_ERR_TIMEOUT.
 struct WaitLimits {
-    long long barrier_clocks;  // grid barrier of the persistent preconditioned solve
+    long long barrier_clocks;  // exchanges of the single-launch loops, grid barrier of the persistent solve
     long long mma_clocks;      // tensor-core completion wait of the network inference
 };
 constexpr long long kDefaultBarrierClocks = 4000000000LL;  // about two seconds

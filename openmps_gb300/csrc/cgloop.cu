@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
     const double thr = S->thr;
     const int max_iter = S->max_iter;
     if (threadIdx.x == 0) {
+        red.wait_clocks = loop_wait_clocks(o);
         sc.rr = S->rr;
         sc.beta = 0.0;
         sc.iter = S->iter;
@@ -236,6 +237,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     if (kCluster) loop_cluster_start();
     LoopSync ls{o.slots, gridDim.x, 0};
     if (threadIdx.x == 0) {
+        red.wait_clocks = loop_wait_clocks(o);
         sc = *o.S;
         alpha32 = __double2float_rn(sc.alpha);
         beta32 = __double2float_rn(sc.beta);
@@ -346,8 +348,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     if (keep) own_rows(o, L, [&](int local, int row) { o.d32[row] = Dv[local]; });
     if (!ok) {
         loop_timeout(o);
-    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *o.S = sc;
+    } else if (blockIdx.x == 0) {
+        store_scalars(o.S, sc);
     }
 }
 

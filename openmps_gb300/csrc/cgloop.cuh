@@ -9,6 +9,8 @@
 // warp had ten.  Blocks with more chunks than the tables hold take them in tiles.
 #pragma once
 
+#include <cstddef>
+
 #include "cg.cuh"
 #include "gridloop.cuh"
 
@@ -291,12 +293,26 @@ __device__ __forceinline__ void own_rows(const CgOperands& o, const LoopView& L,
     }
 }
 
-// a wait of loop_reduce ran out: the step reports it
+// The bound of the loop's waits, by thread 0 before the first exchange.
+__device__ __forceinline__ long long loop_wait_clocks(const CgOperands& o) {
+    return o.limits ? o.limits->barrier_clocks : kDefaultBarrierClocks;
+}
+
+// A wait of loop_reduce ran out: the call reports it, and what the loop leaves counts as not
+// converged (the FP64 CG finishes a mixed-precision solve).
 __device__ __forceinline__ void loop_timeout(const CgOperands& o) {
     if (threadIdx.x == 0) {
         if (o.status) atomicOr(&const_cast<DevStatus*>(o.status)->flags, kStatusWaitTimeout);
-        o.S->aborted = 1;
+        o.S->timed_out = 1;
     }
+}
+
+// The loop's scalars into the solve's, but for timed_out: any block may have set that.
+__device__ __forceinline__ void store_scalars(CgScalars* S, const CgScalars& sc) {
+    constexpr int kWords = static_cast<int>(offsetof(CgScalars, timed_out) / sizeof(uint32_t));
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(&sc);
+    uint32_t* to = reinterpret_cast<uint32_t*>(S);
+    for (int k = static_cast<int>(threadIdx.x); k < kWords; k += static_cast<int>(blockDim.x)) to[k] = from[k];
 }
 
 }  // namespace

@@ -20,8 +20,10 @@
 // totals (divisions) on one thread.  (The sums in fixed point on the integer pipe, limbs added
 // by redux.sync and correctly rounded, took 900 cycles a warp and were dropped.)
 //
-// The grid form's wait is bounded by kLoopWaitClocks: a wait that runs out makes every block
-// leave its loop (the others' waits run out too) with loop_reduce returning false.
+// The grid form's wait is bounded (LoopReduce::wait_clocks): a block whose wait runs out gets
+// false and leaves its loop, and so do the others at the next exchange, where its arrival is
+// missing.  At a loop's last exchange the others may pass: what a block reports then stands
+// beside their result (CgScalars::timed_out).
 #pragma once
 
 #include "common.cuh"
@@ -32,7 +34,7 @@ constexpr int kLoopThreads = 512;  // one block per SM, 128 registers a thread
 constexpr int kLoopMaxBlocks = 256;
 constexpr int kLoopMaxValues = 3;
 constexpr int kLoopCluster = 16;                     // blocks of the cluster form
-constexpr long long kLoopWaitClocks = 4000000000LL;  // about two seconds
+constexpr long long kLoopWaitClocks = 4000000000LL;  // default bound of a wait, about two seconds
 // global words of the grid form: the arrival counter (zeroed by clear_slots in a kernel
 // before the loop), then two sets of partial sums used in turn (a set is written again two
 // rounds later, when every block has arrived at the round between and so has read it)
@@ -44,6 +46,7 @@ struct LoopReduce {
     double cluster[2][kLoopMaxValues][kLoopCluster];
     double warps[kLoopMaxValues][4];
     double total[kLoopMaxValues];
+    long long wait_clocks;  // bound of the grid form's wait, set and read by thread 0
 };
 
 struct LoopSync {
@@ -131,7 +134,7 @@ __device__ __forceinline__ bool loop_reduce(LoopSync& ls, LoopReduce& sh, const 
             while (true) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
                 if (static_cast<int>(seen - ls.arrived) >= 0) break;
-                if (clock64() - t0 > kLoopWaitClocks) {
+                if (clock64() - t0 >= sh.wait_clocks) {
                     late = 1;
                     break;
                 }

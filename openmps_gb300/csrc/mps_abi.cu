@@ -594,6 +594,7 @@ CgOperands cg_operands(mps_handle* h) {
     o.loop_w = h->loop_w;
     o.S = h->S;
     o.status = h->st.status;
+    o.limits = h->d_limits;
     return o;
 }
 
@@ -777,6 +778,7 @@ void do_solve(mps_handle* h) {
         launched(h, 1);
         fb = cg_operands(h);
         fb.S = h->S_fb;
+        fb.limits = nullptr;  // it finishes what a wait under the handle's bound gave up
     }
     if (h->prm.cg_launch == MPS_CG_LAUNCH_HOST) {
         int64_t k = 0;

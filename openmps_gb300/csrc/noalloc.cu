@@ -186,6 +186,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_na_solve(CsrSystem A) {
     if (kCluster) loop_cluster_start();
     LoopSync ls{A.slots, gridDim.x, 0};
     const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
+    if (t == 0) red.wait_clocks = kLoopWaitClocks;
     {
         const int64_t nnz = A.rp[A.n] - A.rp[0];
         const int64_t a = max(static_cast<int64_t>(1), nnz / (4 * static_cast<int64_t>(A.n)));

@@ -114,6 +114,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
     }
     if (lane == 31) wsum[warp] = ws;
     if (t == 0) {
+        red.wait_clocks = loop_wait_clocks(o);
         sc = *o.S;
         first_cell = 0x7fffffff;
         last_cell = -1;
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
         const float* const Dv = vec[2];
         for (int i = r0 + t; i < r1; i += nt) o.x[i] = sc.converged ? xc[i] : xc[i] + static_cast<double>(Dv[i]);
     }
-    if (blockIdx.x == 0 && t == 0) *o.S = sc;
+    if (blockIdx.x == 0) store_scalars(o.S, sc);
 }
 
 int g_pcg_sms = 0;       // SMs of the device (one block each), set by pcg_loop_prepare_device

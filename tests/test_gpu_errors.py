@@ -97,3 +97,39 @@ def test_bounded_wait_runs_out(gpu_lib, which):
         c.forward_time(s.meta["dt"])
     st = c.stats()
     assert st["fallback"] == 0 and st["cg_true_relres"] <= 1e-10
+
+
+@pytest.mark.parametrize("solver", ["cg64", "mixed", "mixed_mg", "learned"])
+def test_loop_wait_runs_out(gpu_lib, solver):
+    # The same bound on the exchanges of the single-launch loops (a scene too large for one
+    # cluster, which waits in hardware): every block but the last to arrive gives up at the
+    # first exchange.  The FP64 CG finishes the mixed-precision solves; a CG64 step ends at
+    # the solve.
+    from openmps_gb300 import learned, scenes
+
+    s = scenes.dam_break(3.2e-3, 0.2, 0.4, 0.8, 0.6)
+    dt = 0.02 * s.l0
+    which = {"cg64": abi.SOLVER_CG64, "mixed": abi.SOLVER_MIXED, "mixed_mg": abi.SOLVER_MIXED_MG,
+             "learned": abi.SOLVER_LEARNED}[solver]
+    c = Computer(s.params(eps=1e-10, solver=which, criterion=abi.CRIT_RHS))
+    if solver == "learned":
+        c.learned_set_weights(learned.load())
+    c.add_scene(s)
+    c.forward_time(dt)
+    c.set_wait_limits(barrier_clocks=0)
+    for _ in range(2):
+        t0 = c.environment().t
+        with pytest.raises(ComputerError) as e:
+            c.forward_time(dt)
+        assert e.value.code == abi.MPS_ERR_TIMEOUT, e.value
+        st = c.stats()
+        if solver != "cg64":
+            assert c.environment().t > t0
+            assert st["fallback"] == 1 and st["cg_true_relres"] <= 1e-10
+        P = c.particles()
+        assert all(np.all(np.isfinite(P[k])) for k in ("x", "z", "u", "w", "p"))
+    c.set_wait_limits()
+    for _ in range(2):
+        c.forward_time(dt)
+        st = c.stats()
+        assert st["fallback"] == 0 and st["cg_true_relres"] <= 1e-10
