@@ -1977,6 +1977,7 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         o.slots = loc.get<double>(kLoopSlots);
         o.loop_w = loc.get<int32_t>(static_cast<size_t>(nchunks));
         o.S = loc.get<CgScalars>(1);
+        o.limits = h->d_limits;
         cudaStream_t s = h->stream;
         check(cudaMemsetAsync(o.tickets, 0, sizeof(uint32_t) * cg_tickets(n), s), "memset");
         auto up = [&](void* d, const void* src, size_t bytes) {
@@ -2005,6 +2006,7 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         if (iterations) *iterations = S.iter;
         if (true_relres) *true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
         h->stats.kernel_launches += 1 + one_launch_count(solver, nullptr, false);
+        if (S.timed_out) throw StatusError{MPS_ERR_TIMEOUT, "a bounded wait of the solve timed out"};
         if (!S.converged)
             throw StatusError{MPS_ERR_CG_NOT_CONVERGED,
                               "Conjugate Gradient method couldn't solve Pressure Poison Equation"};

@@ -173,3 +173,21 @@ def test_empty_rows(gpu_lib, name, solver):
         with pytest.raises(ComputerError) as e:
             c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, max_iters=200, solver=which)
         assert e.value.code == abi.MPS_ERR_CG_NOT_CONVERGED
+
+
+@pytest.mark.parametrize("solver", ["cg64", "mixed"])
+def test_wait_runs_out(gpu_lib, solver):
+    # a bound of 0 cycles: the blocks that arrive first leave the loop, and the call says so
+    from openmps_gb300.computer import Computer, ComputerError
+
+    ptr, col, val, b, xs, x0 = _system(20_000, (1, 2, 140, 141), seed=5)
+    c = Computer(abi.make_params())
+    which = abi.SOLVER_CG64 if solver == "cg64" else abi.SOLVER_MIXED
+    c.set_wait_limits(barrier_clocks=0)
+    with pytest.raises(ComputerError) as e:
+        c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    assert e.value.code == abi.MPS_ERR_TIMEOUT
+    c.set_wait_limits()
+    x, _, rel = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    assert rel <= 1.01e-12
+    assert np.linalg.norm(x - xs) <= TOL * np.linalg.norm(xs)
