@@ -356,13 +356,23 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
  * context may load the library's module and should come before any stream capture.
  * Every call shares the one array: calls that overlap on the GPU (other streams or
  * host threads at the same time) race.  The call returns when the solve is complete.
- * NULL pointers return MPS_ERR_INVALID_ARGUMENT.
+ * NULL pointers return MPS_ERR_INVALID_ARGUMENT.  A grid-wide exchange that waits longer
+ * than about two seconds ends the call with MPS_ERR_TIMEOUT (x is then unspecified).
  * ---------------------------------------------------------------------- */
 #define MPS_NOALLOC_MAX_ROWS 262144
 int mps_cg_solve_csr_device_noalloc(int64_t n, const int64_t* row_ptr, const int32_t* col,
                                     const double* val, const double* b, double* x, double eps,
                                     int32_t criterion, int32_t max_iters, void* stream,
                                     int32_t* iterations, double* true_relres);
+/* The same with the bound of each exchange's wait in SM clock cycles (negative: the
+ * default, 4e9; 0: every wait gives up at its first check), which tests use to let one
+ * run out.  Up to 2,048 rows the exchanges are a cluster's hardware barriers and have no
+ * such wait. */
+int mps_debug_cg_solve_csr_noalloc_wait(int64_t n, const int64_t* row_ptr, const int32_t* col,
+                                        const double* val, const double* b, double* x, double eps,
+                                        int32_t criterion, int32_t max_iters, void* stream,
+                                        int32_t* iterations, double* true_relres,
+                                        int64_t wait_clocks);
 
 /* ------------------------------------------------------------ learned solve
  * No counterpart in the reference (its CG is unpreconditioned and starts from the

@@ -89,6 +89,8 @@ PROTOTYPES = {
                                    C.c_int32, C.c_int32, _I32, _D]),
     "mps_cg_solve_csr_device_noalloc": (C.c_int, [C.c_int64, _P, _P, _P, _P, _P, C.c_double,
                                                   C.c_int32, C.c_int32, _P, _I32, _D]),
+    "mps_debug_cg_solve_csr_noalloc_wait": (C.c_int, [C.c_int64, _P, _P, _P, _P, _P, C.c_double,
+                                                      C.c_int32, C.c_int32, _P, _I32, _D, C.c_int64]),
     "mps_learned_set_weights": (C.c_int, [_P, _F, C.c_int64]),
     "mps_learned_collect": (C.c_int, [_P, C.c_int32]),
     "mps_learned_samples": (C.c_int, [_P, _F, _I32, C.c_int64, _I64]),

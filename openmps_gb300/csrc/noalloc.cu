@@ -73,6 +73,7 @@ struct CsrSystem {
     double eps;
     int criterion, max_iter;
     int keep_rows;  // rows whose vectors fit the block's shared memory
+    long long wait_clocks;  // bound of an exchange's wait
 };
 
 // How a block's warps walk its rows: LANES lanes share a row, GROUPS row groups of a warp at
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_na_solve(CsrSystem A) {
     if (kCluster) loop_cluster_start();
     LoopSync ls{A.slots, gridDim.x, 0};
     const int t = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
-    if (t == 0) red.wait_clocks = kLoopWaitClocks;
+    if (t == 0) red.wait_clocks = A.wait_clocks;
     {
         const int64_t nnz = A.rp[A.n] - A.rp[0];
         const int64_t a = max(static_cast<int64_t>(1), nnz / (4 * static_cast<int64_t>(A.n)));
@@ -360,12 +361,12 @@ cudaError_t launch_na_solve(CsrSystem& A, cudaStream_t s) {
 
 }  // namespace mpsgb
 
-extern "C" int mps_cg_solve_csr_device_noalloc(int64_t n, const int64_t* row_ptr,
-                                               const int32_t* col, const double* val,
-                                               const double* b, double* x, double eps,
-                                               int32_t criterion, int32_t max_iters,
-                                               void* stream, int32_t* iterations,
-                                               double* true_relres) {
+extern "C" int mps_debug_cg_solve_csr_noalloc_wait(int64_t n, const int64_t* row_ptr,
+                                                  const int32_t* col, const double* val,
+                                                  const double* b, double* x, double eps,
+                                                  int32_t criterion, int32_t max_iters,
+                                                  void* stream, int32_t* iterations,
+                                                  double* true_relres, int64_t wait_clocks) {
     using namespace mpsgb;
     if (n <= 0 || !row_ptr || !col || !val || !b || !x) return MPS_ERR_INVALID_ARGUMENT;
     if (n > kNoallocMaxRows) return MPS_ERR_NOALLOC_TOO_LARGE;
@@ -389,6 +390,7 @@ extern "C" int mps_cg_solve_csr_device_noalloc(int64_t n, const int64_t* row_ptr
     A.eps = eps;
     A.criterion = criterion;
     A.max_iter = max_iters > 0 ? max_iters : static_cast<int>(n);
+    A.wait_clocks = wait_clocks < 0 ? kLoopWaitClocks : wait_clocks;
     // the arrival counter starts from zero on every call
     NoallocScalars S{};
     if (cudaMemsetAsync(A.slots, 0, sizeof(double), s) != cudaSuccess || launch_na_solve(A, s) != cudaSuccess ||
@@ -401,4 +403,14 @@ extern "C" int mps_cg_solve_csr_device_noalloc(int64_t n, const int64_t* row_ptr
     if (iterations) *iterations = S.iter;
     if (true_relres) *true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
     return S.converged ? MPS_OK : MPS_ERR_CG_NOT_CONVERGED;
+}
+
+extern "C" int mps_cg_solve_csr_device_noalloc(int64_t n, const int64_t* row_ptr,
+                                               const int32_t* col, const double* val,
+                                               const double* b, double* x, double eps,
+                                               int32_t criterion, int32_t max_iters,
+                                               void* stream, int32_t* iterations,
+                                               double* true_relres) {
+    return mps_debug_cg_solve_csr_noalloc_wait(n, row_ptr, col, val, b, x, eps, criterion, max_iters, stream,
+                                               iterations, true_relres, -1);
 }

@@ -103,3 +103,24 @@ def test_noalloc_rejects_bad_arguments(gpu_lib):
         rc = gpu_lib.mps_cg_solve_csr_device_noalloc(16, *ptrs, 1e-8, abi.CRIT_RHS, 0, None, None,
                                                      None)
         assert rc == abi.MPS_ERR_INVALID_ARGUMENT, ptrs
+
+
+def test_noalloc_wait_runs_out(gpu_lib):
+    # a bound of 0 cycles on a system past the cluster form: the blocks that arrive first
+    # give up and the call says so; the next call with the default bound solves
+    torch = pytest.importorskip("torch")
+    n = 20_000
+    i = np.arange(n)
+    col = np.stack([(i - 1) % n, i, (i + 1) % n], 1).astype(np.int32)
+    val = np.tile([-1.0, 3.0, -1.0], (n, 1))
+    xs = np.random.default_rng(1).standard_normal(n)
+    b = (val * xs[col]).sum(1)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in
+           (np.arange(0, 3 * n + 1, 3, dtype=np.int64), col.ravel(), val.ravel(), b)]
+    for wait, want in ((0, abi.MPS_ERR_TIMEOUT), (-1, abi.MPS_OK), (0, abi.MPS_ERR_TIMEOUT), (-1, abi.MPS_OK)):
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        rc = gpu_lib.mps_debug_cg_solve_csr_noalloc_wait(n, *[d.data_ptr() for d in dev], x.data_ptr(), 1e-12,
+                                                         abi.CRIT_RHS, 0, None, None, None, wait)
+        assert rc == want
+    # condition number 5, |b - A x| <= 1e-12 |b|
+    assert np.linalg.norm(x.cpu().numpy() - xs) <= 1e-11 * np.linalg.norm(xs)
