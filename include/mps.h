@@ -356,6 +356,9 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
  * context may load the library's module and should come before any stream capture.
  * Every call shares the one array: calls that overlap on the GPU (other streams or
  * host threads at the same time) race.  The call returns when the solve is complete.
+ * Past 2,048 rows the solve is one cooperative launch with a block on every SM that the
+ * stream can use (a green context's stream: on its SMs): it starts when each has room, and
+ * other work on those SMs waits while it runs.
  * NULL pointers return MPS_ERR_INVALID_ARGUMENT.  A grid-wide exchange that waits longer
  * than about two seconds ends the call with MPS_ERR_TIMEOUT (x is then unspecified).
  * ---------------------------------------------------------------------- */

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     }
 }
 
-int g_loop_sms = 0;        // SMs of the device (one block each), set by cg_loop_prepare_device
+int g_loop_sms = 0;        // blocks of the grid form, set by cg_loop_prepare_device
 int g_loop_cluster = 0;    // blocks of the cluster form (0: a cluster of that size cannot run)
 size_t g_loop_smem = 0;    // largest dynamic shared memory of a block
 
@@ -409,7 +409,7 @@ cudaError_t launch_loop(void (*kernel)(CgOperands, LoopPlan), const CgOperands& 
         at[0].val.cooperative = 1;
     }
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p.blocks > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, o, p);
 }
 
@@ -432,7 +432,8 @@ cudaError_t cg_loop_prepare_device() {
         if (e != cudaSuccess) return e;
     }
     g_loop_smem = room;
-    g_loop_sms = sms < kLoopMaxBlocks ? sms : kLoopMaxBlocks;
+    e = loop_grid_blocks(dev, sms, &g_loop_sms);
+    if (e != cudaSuccess) return e;
     int cluster = kLoopCluster;
     for (auto k : {k_cg_loop<true>, k_mx_loop<true>}) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);

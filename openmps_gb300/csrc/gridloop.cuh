@@ -55,6 +55,15 @@ struct LoopSync {
     int round;         // 0, 1, 0, ...
 };
 
+// Blocks of the grid form on `sms` SMs: one each where the device launches cooperatively (all
+// blocks of a launch must be resident at once), else a single one, which waits for nobody.
+inline cudaError_t loop_grid_blocks(int dev, int sms, int* blocks) {
+    int coop = 0;
+    const cudaError_t e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    *blocks = !coop ? 1 : sms < kLoopMaxBlocks ? sms : kLoopMaxBlocks;
+    return e;
+}
+
 // Readies the slots for the loop kernel launched after this one (any grid).
 __device__ __forceinline__ void clear_slots(double* slots) {
     if (slots && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned*>(slots) = 0u;

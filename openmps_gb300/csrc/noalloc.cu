@@ -34,6 +34,8 @@
 // takes a warp-wide addition every 64 cycles).  Before, one thread walked a row (a warp's
 // loads touched 32 rows apart) in three kernels per iteration, and the host read the
 // convergence flag every 16 iterations.
+#include <cuda.h>
+
 #include <cmath>
 
 #include "gridloop.cuh"
@@ -314,15 +316,46 @@ int scratch_for_current_context(double** out) {
     return MPS_OK;
 }
 
+// SMs that work on the stream can use: `sms` (the device's), or the part that the stream's
+// green context has.
+int stream_sms(cudaStream_t s, int sms) {
+    auto entry = [](const char* name, unsigned version) {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return static_cast<void*>(nullptr);
+        }
+        return f;
+    };
+    static const auto stream_ctx = reinterpret_cast<CUresult (*)(CUstream, CUcontext*)>(entry("cuStreamGetCtx", 9020));
+    static const auto resource = reinterpret_cast<CUresult (*)(CUcontext, CUdevResource*, CUdevResourceType)>(
+        entry("cuCtxGetDevResource", 12040));
+    CUcontext ctx = nullptr;
+    CUdevResource r{};
+    if (!stream_ctx || !resource || stream_ctx(s, &ctx) != CUDA_SUCCESS ||
+        resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return sms;
+    const int part = static_cast<int>(r.sm.smCount);
+    return part > 0 && part < sms ? part : sms;
+}
+
 // One cluster for small systems, else a block per SM; p, s, x, r of half as many rows again
-// as the average block owns in shared memory.
+// as the average block owns in shared memory.  All blocks must be resident at once: on a
+// stream with a part of the SMs the grid is as many blocks as that part has (the blocks'
+// shares of the rows follow from the grid; a cluster's 16 SMs must lie in one cluster of
+// the chip, which a part need not have).
 cudaError_t launch_na_solve(CsrSystem& A, cudaStream_t s) {
-    int dev = 0, sms = 0, most = 0;
+    int dev = 0, all = 0, most = 0, grid = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&all, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    bool cluster = A.n <= kNoallocClusterRows;
+    const int sms = stream_sms(s, all);
+    e = loop_grid_blocks(dev, sms, &grid);
+    if (e != cudaSuccess) return e;
+    bool cluster = A.n <= kNoallocClusterRows && sms == all;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     cfg.blockDim = dim3(kLoopThreads);
@@ -331,7 +364,7 @@ cudaError_t launch_na_solve(CsrSystem& A, cudaStream_t s) {
     cfg.numAttrs = 1;
     for (;; cluster = false) {
         auto kernel = cluster ? k_na_solve<true> : k_na_solve<false>;
-        const int blocks = cluster ? kLoopCluster : (sms < kLoopMaxBlocks ? sms : kLoopMaxBlocks);
+        const int blocks = cluster ? kLoopCluster : grid;
         const int64_t room = (most - 16 * 1024) / (4 * static_cast<int64_t>(sizeof(double)));
         const int64_t want = 3 * static_cast<int64_t>(A.n) / (2 * blocks) + 128;
         A.keep_rows = static_cast<int>(want < room ? want : room);
@@ -343,7 +376,12 @@ cudaError_t launch_na_solve(CsrSystem& A, cudaStream_t s) {
         if (!cluster) {
             at[0].id = cudaLaunchAttributeCooperative;
             at[0].val.cooperative = 1;
-            return cudaLaunchKernelEx(&cfg, kernel, A);
+            cfg.numAttrs = blocks > 1 ? 1 : 0;
+            e = cudaLaunchKernelEx(&cfg, kernel, A);
+            if (e != cudaErrorCooperativeLaunchTooLarge || blocks == 1) return e;
+            cudaGetLastError();  // fewer SMs than the device and the stream report
+            grid = blocks / 2;
+            continue;
         }
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = kLoopCluster;

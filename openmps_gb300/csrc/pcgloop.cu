@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pcg_loop(CgOperands o, MgHi
     if (blockIdx.x == 0) store_scalars(o.S, sc);
 }
 
-int g_pcg_sms = 0;       // SMs of the device (one block each), set by pcg_loop_prepare_device
+int g_pcg_sms = 0;       // blocks of the grid form, set by pcg_loop_prepare_device
 bool g_pcg_cluster = false;
 size_t g_pcg_smem = 0;   // largest dynamic shared memory of a block
 
@@ -605,7 +605,8 @@ cudaError_t pcg_loop_prepare_device() {
     e = cudaFuncSetAttribute(k_pcg_loop<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     g_pcg_smem = room;
-    g_pcg_sms = sms < kLoopMaxBlocks ? sms : kLoopMaxBlocks;
+    e = loop_grid_blocks(dev, sms, &g_pcg_sms);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kLoopCluster);
     cfg.blockDim = dim3(kLoopThreads);
@@ -648,7 +649,7 @@ cudaError_t launch_pcg_loop(const CgOperands& o, const MgHierarchy& mg, cudaStre
         at[0].val.cooperative = 1;
     }
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = p.blocks > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, cluster ? k_pcg_loop<true> : k_pcg_loop<false>, o, mg, p);
 }
 

@@ -124,3 +124,55 @@ def test_noalloc_wait_runs_out(gpu_lib):
         assert rc == want
     # condition number 5, |b - A x| <= 1e-12 |b|
     assert np.linalg.norm(x.cpu().numpy() - xs) <= 1e-11 * np.linalg.norm(xs)
+
+
+class _GreenStream:
+    """A stream of a green context with `sms` SMs (CUDA driver API; of this process only)."""
+
+    def __init__(self, sms):
+        self.cu = C.CDLL("libcuda.so.1")
+        box = lambda: C.create_string_buffer(512)  # a CUdevResource, with room to spare
+        self.ctx, self.stream = C.c_void_p(), C.c_void_p()
+        dev, whole, part, rest, desc = C.c_int(), box(), box(), box(), C.c_void_p()
+        groups = C.c_uint(1)
+        self._ok("cuDeviceGet", C.byref(dev), 0)
+        self._ok("cuDeviceGetDevResource", dev, whole, 1)  # 1: SMs
+        self._ok("cuDevSmResourceSplitByCount", part, C.byref(groups), whole, rest, 0, sms)
+        self._ok("cuDevResourceGenerateDesc", C.byref(desc), part, 1)
+        self._ok("cuGreenCtxCreate", C.byref(self.ctx), desc, dev, 1)  # 1: default stream
+        self._ok("cuGreenCtxStreamCreate", C.byref(self.stream), self.ctx, 1, 0)  # 1: non-blocking
+
+    def _ok(self, name, *args):
+        rc = getattr(self.cu, name)(*args)
+        assert rc == 0, (name, rc)
+
+    def close(self):
+        self._ok("cuStreamDestroy_v2", self.stream)
+        self._ok("cuGreenCtxDestroy", self.ctx)
+
+
+@pytest.mark.parametrize("n", [500, 2048, 2049, 20_000, 100_003])
+def test_noalloc_on_a_part_of_the_chip(gpu_lib, n):
+    # on a stream with a part of the SMs the solve's grid is as large as that part
+    torch = pytest.importorskip("torch")
+    i = np.arange(n)
+    col = np.stack([(i - 1) % n, i, (i + 1) % n], 1).astype(np.int32)
+    val = np.tile([-1.0, 3.0, -1.0], (n, 1))
+    xs = np.random.default_rng(1).standard_normal(n)
+    b = (val * xs[col]).sum(1)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in
+           (np.arange(0, 3 * n + 1, 3, dtype=np.int64), col.ravel(), val.ravel(), b)]
+    torch.cuda.synchronize()
+    g = _GreenStream(32)
+    got = []
+    for stream in (g.stream, None, g.stream):
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        rc = gpu_lib.mps_cg_solve_csr_device_noalloc(n, *[d.data_ptr() for d in dev], x.data_ptr(), 1e-12,
+                                                     abi.CRIT_RHS, 0, stream, None, None)
+        assert rc == abi.MPS_OK
+        got.append(x.cpu().numpy())
+        # condition number 5, |b - A x| <= 1e-12 |b|
+        assert np.linalg.norm(got[-1] - xs) <= 1e-11 * np.linalg.norm(xs)
+    g.close()
+    assert np.array_equal(got[0], got[2])
