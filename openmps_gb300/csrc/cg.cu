@@ -1323,10 +1323,11 @@ cudaError_t one_launch_kernels(int solver, const CgOperands& ops, cudaStream_t s
 }
 }  // namespace
 
-int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb) {
-    const int tail = with_fb ? 4 : 1;  // the fallback's init, loop and merge; the true residual
-    if (solver == MPS_SOLVER_CG64) return 2 + 1;
-    if (solver == MPS_SOLVER_MIXED) return 4 + tail;
+int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb, int nchunks) {
+    const int loop = cg_loop_launches(nchunks);
+    const int tail = with_fb ? 3 + loop : 1;  // the fallback's init, loop and merge; the true residual
+    if (solver == MPS_SOLVER_CG64) return 1 + loop + 1;
+    if (solver == MPS_SOLVER_MIXED) return 3 + loop + tail;
     const bool learned = solver == MPS_SOLVER_LEARNED;
     return mg_setup_launches(*mg, learned) + 2 + tail + (learned ? 1 + learned_prep_launches(*mg, true) : 0);
 }
@@ -1575,7 +1576,7 @@ cudaError_t cg_run_direct(int solver, const CgOperands& ops, CgScalars* host_S, 
     if (solver == MPS_SOLVER_LEARNED && !lrn) return cudaErrorInvalidValue;
     if (loops_in_one_launch(solver, mg)) {
         const cudaError_t e = one_launch_kernels(solver, ops, s, mg, fb, lrn, nullptr);
-        if (launches) *launches = one_launch_count(solver, mg, fb != nullptr);
+        if (launches) *launches = one_launch_count(solver, mg, fb != nullptr, ops.nchunks);
         return e == cudaSuccess ? cudaGetLastError() : e;
     }
     const cudaGraphConditionalHandle none = 0;

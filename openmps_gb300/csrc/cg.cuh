@@ -202,10 +202,12 @@ struct LearnedOps;
 constexpr int kMixedStallIter = 2000;
 
 // cgloop.cu: the iteration loops of MPS_SOLVER_CG64 (after k_cg_init) and MPS_SOLVER_MIXED
-// (after k_mx_init and the first k_mx_spmv), one cooperative launch each.
+// (after k_mx_init and the first k_mx_spmv), one launch each, a cluster or a cooperative
+// grid; past the sizes that a block's tables surely hold two, of which one returns at once.
 cudaError_t launch_cg_loop(const CgOperands& o, cudaStream_t s);
 cudaError_t launch_mx_loop(const CgOperands& o, cudaStream_t s);
 cudaError_t cg_loop_prepare_device();
+int cg_loop_launches(int nchunks);
 
 // Bounds of the device-side waits, in SM clock cycles, kept in device memory per handle
 // so that captured graphs read the current values.  A wait gives up once this many
@@ -299,7 +301,7 @@ cudaError_t cg_run_direct(int solver, const CgOperands& ops, CgScalars* host_S, 
 // Grid size of the persistent solve on the current device (0: cooperative launch unavailable).
 int persistent_blocks();
 // Kernels of a solve whose loop is one launch (with_fb: and the fallback's).
-int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb);
+int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb, int nchunks);
 
 // Sets eps / criterion / max_iter / delta for the next solve (stream-ordered).
 void launch_cg_configure(CgScalars* S, double eps, int criterion, int max_iter, double delta2,

@@ -20,14 +20,13 @@ namespace mpsgb {
 
 namespace {
 
-constexpr int kTileChunks = 128;  // of a block whose chunks pass the tables
-
 // dynamic shared memory: unit sums, tables, vectors.  (The gathered vector's rows around the
 // block in shared memory too were measured: 42,226 rows 13.0 against 12.4 us, 90,050 rows
 // 18.8 against 18.4, MIXED 13.9 against 14.0: loading them costs what the gathers wait.)
 struct LoopPlan {
     int blocks;
-    int tables;      // chunks the tables hold: all that a block can own, or one tile
+    int tables;      // chunks the tables hold
+    bool either;     // the direct form follows, for systems whose chunks in the loop pass them
     int keep_bytes;  // shared memory for the block's vectors
     size_t smem;
 };
@@ -41,6 +40,7 @@ size_t table_bytes(int tables) {
 // floor(P_k G / P_N), P_k = (widths before it) + a (chunks before it), a = W / (4 N) (a
 // row's vector work is about ten matrix entries' at the 46 entries of the usual radius): a
 // block then owns at most 5 N / G + 1 chunks, and even shares when the widths are alike.
+template <bool kDirect>
 __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPlan& plan, unsigned char* sm,
                                              unsigned char** keep) {
     __shared__ int wsum[32], wcnt[32], first_pos, last_pos, first_chunk, last_chunk;
@@ -84,6 +84,10 @@ __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPla
         W += wsum[k];
         N += wcnt[k];
     }
+    if (plan.either && (2 * (N / static_cast<int>(gridDim.x) + 1) + 2 > plan.tables) != kDirect) {
+        L.nc = -1;  // the other form's (every block finds the same)
+        return L;
+    }
     const long long a = N > 0 ? max(1, W / (4 * N)) : 1;
     const long long total = W + a * N;
     const long long G = gridDim.x;
@@ -108,9 +112,9 @@ __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPla
         __syncthreads();
         if (pass == 0) {
             const int mine = last_pos < 0 ? 0 : last_pos - first_pos + 1;
-            L.whole = mine <= plan.tables;
-            L.c0 = L.whole ? 0 : first_chunk;
-            L.nc = L.whole ? mine : last_chunk - first_chunk + 1;
+            L.whole = !kDirect && mine <= plan.tables;
+            L.c0 = L.whole || mine == 0 ? 0 : first_chunk;
+            L.nc = L.whole || mine == 0 ? mine : last_chunk - first_chunk + 1;
         }
     }
     split_tiles(L, plan.tables);
@@ -118,7 +122,7 @@ __device__ __forceinline__ LoopView loop_view(const CgOperands& o, const LoopPla
     return L;
 }
 
-template <bool kCluster>
+template <bool kCluster, bool kDirect>
 __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopPlan plan) {
     extern __shared__ __align__(16) unsigned char loop_sm[];
     __shared__ LoopReduce red;
@@ -129,7 +133,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
     CgScalars* S = o.S;
     if (S->converged || S->aborted || S->iter >= S->max_iter) return;
     unsigned char* keep_sm;
-    const LoopView L = loop_view(o, plan, loop_sm, &keep_sm);
+    const LoopView L = loop_view<kDirect>(o, plan, loop_sm, &keep_sm);
+    if (L.nc < 0) return;
     if (kCluster) loop_cluster_start();
     LoopSync ls{o.slots, gridDim.x, 0};
     const double thr = S->thr;
@@ -144,13 +149,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
     // the block's rows of p, s, x and r: index `a` of a row is its place in the block when
     // they are kept in shared memory, the row itself in the global arrays
     const int rows = L.nc * kSellRows;
-    const bool keep = L.whole && 4 * static_cast<int64_t>(sizeof(double)) * rows <= plan.keep_bytes;
+    const bool keep = !kDirect && L.whole && 4 * static_cast<int64_t>(sizeof(double)) * rows <= plan.keep_bytes;
     double* kept = reinterpret_cast<double*>(keep_sm);
     double* P = keep ? kept : o.p;
     double* Q = keep ? kept + rows : o.Ap;
     double* X = keep ? kept + 2 * rows : o.x;
     double* R = keep ? kept + 3 * rows : o.r;
-    own_rows(o, L, [&](int local, int row) {
+    own_rows<kDirect>(o, L, [&](int local, int row) {
         const int a = keep ? local : row;
         P[a] = 0.0;
         Q[a] = 0.0;
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
         double v = 0.0;
         {
             const double beta = sc.beta;
-            product<double>(o, L, [&](int j) { return o.r[j]; }, [&](int local, int row, double ar) {
+            product<double, kDirect>(o, L, [&](int j) { return o.r[j]; }, [&](int local, int row, double ar) {
                 const int a = keep ? local : row;
                 const double p = fma(beta, P[a], R[a]);
                 const double s = fma(beta, Q[a], ar);
@@ -187,7 +192,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
         v = 0.0;
         {
             const double alpha = sc.alpha;
-            own_rows(o, L, [&](int local, int row) {
+            own_rows<kDirect>(o, L, [&](int local, int row) {
                 const int a = keep ? local : row;
                 X[a] = fma(alpha, P[a], X[a]);
                 const double ri = fma(-alpha, Q[a], R[a]);
@@ -211,7 +216,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
         });
         if (ok && (sc.conv || sc.iter >= max_iter)) break;
     }
-    if (keep) own_rows(o, L, [&](int local, int row) { o.x[row] = X[local]; });
+    if (keep) own_rows<kDirect>(o, L, [&](int local, int row) { o.x[row] = X[local]; });
     if (!ok) {
         loop_timeout(o);
     } else if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(CgOperands o, LoopP
     }
 }
 
-template <bool kCluster>
+template <bool kCluster, bool kDirect>
 __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopPlan plan) {
     extern __shared__ __align__(16) unsigned char loop_sm[];
     __shared__ LoopReduce red;
@@ -233,7 +238,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     __shared__ float alpha32, beta32;
     if (o.S->converged || o.S->aborted || o.S->iter >= o.S->max_iter) return;
     unsigned char* keep_sm;
-    const LoopView L = loop_view(o, plan, loop_sm, &keep_sm);
+    const LoopView L = loop_view<kDirect>(o, plan, loop_sm, &keep_sm);
+    if (L.nc < 0) return;
     if (kCluster) loop_cluster_start();
     LoopSync ls{o.slots, gridDim.x, 0};
     if (threadIdx.x == 0) {
@@ -244,7 +250,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     }
     // the block's rows of s, p, d, w and r (kept or global, as in k_cg_loop)
     const int rows = L.nc * kSellRows;
-    const bool keep = L.whole && 5 * static_cast<int64_t>(sizeof(float)) * rows <= plan.keep_bytes;
+    const bool keep = !kDirect && L.whole && 5 * static_cast<int64_t>(sizeof(float)) * rows <= plan.keep_bytes;
     float* kept = reinterpret_cast<float*>(keep_sm);
     float* Sv = keep ? kept : o.s32;
     float* Pv = keep ? kept + rows : o.p32;
@@ -252,7 +258,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     float* Wv = keep ? kept + 3 * rows : o.w32;
     float* Rv = keep ? kept + 4 * rows : o.r32;
     if (keep)
-        own_rows(o, L, [&](int local, int row) {
+        own_rows<kDirect>(o, L, [&](int local, int row) {
             Sv[local] = o.s32[row];
             Pv[local] = o.p32[row];
             Dv[local] = o.d32[row];
@@ -263,7 +269,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
     // w = A r (FP32); gamma = r.r and delta = w.r in FP64, and what follows from them
     auto spmv = [&](bool after_update) {
         double v[2] = {0.0, 0.0};
-        product<float>(o, L, [&](int j) { return o.r32[j]; }, [&](int local, int row, float w) {
+        product<float, kDirect>(o, L, [&](int j) { return o.r32[j]; }, [&](int local, int row, float w) {
             const int a = keep ? local : row;
             const double ri = widen(Rv[a]);
             Wv[a] = w;
@@ -303,7 +309,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
         {
             // s = w + beta s; p = r + beta p; d += alpha p; r -= alpha s
             const float alpha = alpha32, beta = beta32;
-            own_rows(o, L, [&](int local, int row) {
+            own_rows<kDirect>(o, L, [&](int local, int row) {
                 const int a = keep ? local : row;
                 const float si = fmaf(beta, Sv[a], Wv[a]);
                 const float pi = fmaf(beta, Pv[a], Rv[a]);
@@ -321,13 +327,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
         const bool odd = (sc.updates & 1) != 0;
         const double* xc = odd ? o.x2 : o.x;
         double* xn = odd ? o.x : o.x2;
-        own_rows(o, L, [&](int local, int row) {
+        own_rows<kDirect>(o, L, [&](int local, int row) {
             xn[row] = xc[row] + static_cast<double>(Dv[keep ? local : row]);
         });
         ok = loop_reduce<kCluster, 0>(ls, red, nullptr, 0, [](const double*) {});
         if (!ok) break;
         double v = 0.0;
-        product<double>(o, L, [&](int j) { return xn[j]; }, [&](int local, int row, double ax) {
+        product<double, kDirect>(o, L, [&](int j) { return xn[j]; }, [&](int local, int row, double ax) {
             const double ri = o.b[row] - ax;
             const float rf = __double2float_rn(ri);
             Rv[keep ? local : row] = rf;
@@ -345,7 +351,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_mx_loop(CgOperands o, LoopP
         if (!ok || sc.converged) break;
         ok = spmv(true);
     }
-    if (keep) own_rows(o, L, [&](int local, int row) { o.d32[row] = Dv[local]; });
+    if (keep) own_rows<kDirect>(o, L, [&](int local, int row) { o.d32[row] = Dv[local]; });
     if (!ok) {
         loop_timeout(o);
     } else if (blockIdx.x == 0) {
@@ -367,6 +373,11 @@ size_t g_loop_smem = 0;    // largest dynamic shared memory of a block
 // (WHILE: 30.4, 31.5, 37.2, 73.7), MIXED 7.7, 9.4, 14.0 (20.6, 21.7, 25.1); the FP64 pipe
 // bounds the large CG64 systems (one multiply-add per entry: 6.4 us at 90,050 rows), the
 // exchanges the small ones.
+// More chunks in the loop than a block's tables hold: whole chunks are walked without tables
+// (kDirect).  CG64 / MIXED, us per iteration, with kernels per phase, with tables built again
+// tile by tile in each product, and walked: 1.69 M rows of 28.9 entries 183 / 116, 170 / 134,
+// 139 / 92; 2.4 M of 13 203 / 125, 176 / 133, 128 / 77; 4 M of 13 273 / 186, 339 / 278,
+// 240 / 107 (DRAM's 6.8 TB/s bound these: 4 M rows are 624 / 416 MB of matrix an iteration).
 constexpr int kClusterChunks64 = 80, kClusterChunks32 = 128;
 
 LoopPlan loop_plan(int nchunks, bool cluster, int keep_row_bytes) {
@@ -375,12 +386,16 @@ LoopPlan loop_plan(int nchunks, bool cluster, int keep_row_bytes) {
     if (!cluster && p.blocks > nchunks) p.blocks = nchunks;
     const int per = (nchunks + p.blocks - 1) / p.blocks;
     // two or three times the average share (a block of thin chunks alone can own five times
-    // it, and then works in tiles)
-    p.tables = kTileChunks;
+    // it, and then works in tiles); where that does not fit, as many as do: what the loop
+    // leaves out (most rows in three dimensions) is known on the device only
     if (table_bytes(3 * per + 2) <= g_loop_smem / 2)
         p.tables = 3 * per + 2;
     else if (table_bytes(2 * per + 2) <= g_loop_smem / 4 * 3)
         p.tables = 2 * per + 2;
+    else {
+        p.either = true;
+        p.tables = static_cast<int>((g_loop_smem / 4 * 3 - table_bytes(0)) / (table_bytes(1) - table_bytes(0)));
+    }
     const size_t left = g_loop_smem - table_bytes(p.tables);
     // half as much again as the average block's vectors (the rest of the SM's memory is L1)
     const size_t want = (static_cast<size_t>(per) * 3 / 2 + 4) * kSellRows * keep_row_bytes;
@@ -389,8 +404,14 @@ LoopPlan loop_plan(int nchunks, bool cluster, int keep_row_bytes) {
     return p;
 }
 
-cudaError_t launch_loop(void (*kernel)(CgOperands, LoopPlan), const CgOperands& o, bool cluster, int keep_row_bytes,
-                        cudaStream_t s) {
+using LoopKernel = void (*)(CgOperands, LoopPlan);
+struct LoopKernels {
+    LoopKernel cluster, grid, direct;
+};
+constexpr LoopKernels kCgLoops{k_cg_loop<true, false>, k_cg_loop<false, false>, k_cg_loop<false, true>};
+constexpr LoopKernels kMxLoops{k_mx_loop<true, false>, k_mx_loop<false, false>, k_mx_loop<false, true>};
+
+cudaError_t launch_loop(const LoopKernels& k, const CgOperands& o, bool cluster, int keep_row_bytes, cudaStream_t s) {
     if (o.nchunks <= 0) return cudaErrorInvalidValue;
     const LoopPlan p = loop_plan(o.nchunks, cluster, keep_row_bytes);
     cudaLaunchConfig_t cfg = {};
@@ -410,7 +431,10 @@ cudaError_t launch_loop(void (*kernel)(CgOperands, LoopPlan), const CgOperands& 
     }
     cfg.attrs = at;
     cfg.numAttrs = p.blocks > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, o, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, cluster ? k.cluster : k.grid, o, p);
+    if (e != cudaSuccess || !p.either) return e;
+    cfg.dynamicSmemBytes = 0;
+    return cudaLaunchKernelEx(&cfg, k.direct, o, p);
 }
 
 }  // namespace
@@ -422,7 +446,7 @@ cudaError_t cg_loop_prepare_device() {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
     size_t room = static_cast<size_t>(most);
-    for (auto k : {k_cg_loop<false>, k_cg_loop<true>, k_mx_loop<false>, k_mx_loop<true>}) {
+    for (auto k : {kCgLoops.cluster, kCgLoops.grid, kCgLoops.direct, kMxLoops.cluster, kMxLoops.grid, kMxLoops.direct}) {
         cudaFuncAttributes a{};
         e = cudaFuncGetAttributes(&a, k);
         if (e != cudaSuccess) return e;
@@ -435,7 +459,7 @@ cudaError_t cg_loop_prepare_device() {
     e = loop_grid_blocks(dev, sms, &g_loop_sms);
     if (e != cudaSuccess) return e;
     int cluster = kLoopCluster;
-    for (auto k : {k_cg_loop<true>, k_mx_loop<true>}) {
+    for (auto k : {kCgLoops.cluster, kMxLoops.cluster}) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
@@ -459,14 +483,18 @@ cudaError_t cg_loop_prepare_device() {
     return cudaSuccess;
 }
 
+int cg_loop_launches(int nchunks) {
+    return nchunks > kClusterChunks32 && loop_plan(nchunks, false, 0).either ? 2 : 1;
+}
+
 cudaError_t launch_cg_loop(const CgOperands& o, cudaStream_t s) {
     const bool cluster = g_loop_cluster > 0 && o.nchunks <= kClusterChunks64;
-    return launch_loop(cluster ? k_cg_loop<true> : k_cg_loop<false>, o, cluster, 4 * sizeof(double), s);
+    return launch_loop(kCgLoops, o, cluster, 4 * sizeof(double), s);
 }
 
 cudaError_t launch_mx_loop(const CgOperands& o, cudaStream_t s) {
     const bool cluster = g_loop_cluster > 0 && o.nchunks <= kClusterChunks32;
-    return launch_loop(cluster ? k_mx_loop<true> : k_mx_loop<false>, o, cluster, 5 * sizeof(float), s);
+    return launch_loop(kMxLoops, o, cluster, 5 * sizeof(float), s);
 }
 
 }  // namespace mpsgb

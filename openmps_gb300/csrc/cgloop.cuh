@@ -6,7 +6,8 @@
 // sums are parked in shared memory and the row's thread adds them.  18 chunks of 41 entries
 // (84k rows over 152 SMs) are 108 steps, seven for each of 16 warps at most; in units of 16
 // entries dealt out whole (MIXED 16.4, CG64 21.9 us an iteration at 90,050 rows) the longest
-// warp had ten.  Blocks with more chunks than the tables hold take them in tiles.
+// warp had ten.  A block with more chunks than its tables hold takes them in tiles; where the
+// blocks' shares pass what tables fit, the loops walk whole chunks without (ChunkCursor).
 #pragma once
 
 #include <cstddef>
@@ -149,7 +150,7 @@ struct UnitStep {
     int c[kStep];
     T a[kStep];
     bool live;  // the lane's row is the block's and has entries
-    int out;    // the unit, when this is its last step (else -1)
+    int out;    // the unit (ChunkCursor: chunk), when this is its last step (else -1)
 };
 
 // The warp's steps in order.  A chunk's entries past a row's length are {the row itself, 0}
@@ -188,8 +189,8 @@ struct UnitCursor {
             s.a[e] = __uint_as_float(p.y);
         }
     }
-    // Loads the current step and moves on.
-    __device__ __forceinline__ void load(UnitStep<T>& s) {
+    // Loads the current step and moves past it.
+    __device__ __forceinline__ void step(UnitStep<T>& s) {
         const int64_t from = at + static_cast<int64_t>(k0) * kSellRows;
         s.live = live;
         s.out = -1;
@@ -205,6 +206,9 @@ struct UnitCursor {
             }
         }
         k0 += kStep;
+    }
+    __device__ __forceinline__ void load(UnitStep<T>& s) {
+        step(s);
         if (k0 >= end) {
             s.out = u++;
             if (u < u1) open();
@@ -212,15 +216,12 @@ struct UnitCursor {
     }
 };
 
-// The unit sums of the tables' chunks: T = double (FP64 matrix) or float (FP32 pairs).  Two
-// steps in turn, each loaded while the other gathers and adds: a warp waits for one round
-// trip to L2 per step (0.6 us across the dies), not for two.
-template <class T, class V>
-__device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L, V v) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    T* part = reinterpret_cast<T*>(L.part);
-    const int2 mine = L.share[warp];
-    UnitCursor<T> cur(o, L, mine.x, mine.y);
+// The sums of a cursor's steps, T = double (FP64 matrix) or float (FP32 pairs): done(out, the
+// lane's sum) at the last step of each unit or chunk.  Two steps in turn, each loaded while
+// the other gathers and adds: a warp waits for one round trip to L2 per step (0.6 us across
+// the dies), not for two.
+template <class T, class Cursor, class V, class D>
+__device__ __forceinline__ void walk_steps(Cursor& cur, V v, D done) {
     if (!cur.valid()) return;
     T acc = 0;
     auto add = [&](const UnitStep<T>& s) {
@@ -235,7 +236,7 @@ __device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L
             }
         }
         if (s.out >= 0) {
-            part[s.out * 32 + lane] = acc;
+            done(s.out, acc);
             acc = 0;
         }
     };
@@ -253,11 +254,80 @@ __device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L
     }
 }
 
+// The unit sums of the tables' chunks.
+template <class T, class V>
+__device__ __forceinline__ void unit_sums(const CgOperands& o, const LoopView& L, V v) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    T* part = reinterpret_cast<T*>(L.part);
+    const int2 mine = L.share[warp];
+    UnitCursor<T> cur(o, L, mine.x, mine.y);
+    walk_steps<T>(cur, v, [&](int unit, T sum) { part[unit * 32 + lane] = sum; });
+}
+
+// The steps of a block without tables: its chunks that the loop works on, dealt to the warps
+// in turn, with a row's sum in its lane's register to the end.  A warp looks 32 of its chunks
+// over at once, and loads the next one's place while the present one is read.
+template <class T>
+struct ChunkCursor : UnitCursor<T> {
+    int k, next;              // the block's chunk, the warp's next one (nc: none)
+    int next_off, next_size;
+    int group;                // first of the chunks not looked over yet
+    unsigned pending;         // chunks of the 32 before them to come
+
+    __device__ __forceinline__ void take() {
+        const int lane = threadIdx.x & 31, w = this->L.warps, nc = this->L.nc;
+        while (pending == 0u) {
+            if (group >= nc) {
+                next = nc;
+                return;
+            }
+            const int q = group + lane * w;
+            pending = __ballot_sync(0xffffffffu, q < nc && this->o.loop_w[this->L.c0 + q] > 0);
+            group += 32 * w;
+        }
+        next = group - 32 * w + (__ffs(static_cast<int>(pending)) - 1) * w;
+        pending &= pending - 1u;
+        next_off = this->o.off[this->L.c0 + next];
+        next_size = this->o.chunk[this->L.c0 + next];
+    }
+    __device__ __forceinline__ void open() {
+        k = next;
+        if (!valid()) return;
+        this->row = (this->L.c0 + k) * kSellRows + static_cast<int>(threadIdx.x & 31);
+        this->at = static_cast<int64_t>(next_off) + (threadIdx.x & 31);
+        this->k0 = 0;
+        this->end = next_size / kSellRows;
+        this->live = this->row >= this->L.lo && this->row < this->L.hi;
+        take();
+    }
+    __device__ __forceinline__ ChunkCursor(const CgOperands& o_, const LoopView& L_)
+        : UnitCursor<T>(o_, L_, 0, 0), next_off(0), next_size(0), group(static_cast<int>(threadIdx.x >> 5)), pending(0u) {
+        take();
+        open();
+    }
+    __device__ __forceinline__ bool valid() const { return k < this->L.nc; }
+    __device__ __forceinline__ void load(UnitStep<T>& s) {
+        this->step(s);
+        if (this->k0 >= this->end) {
+            s.out = k;
+            open();
+        }
+    }
+};
+
 // f(local row, row, (A v)_row) for every row of the block, by the row's thread; v(column)
-// gathers the vector
-template <class T, class V, class F>
+// gathers the vector (kDirect: a block without tables)
+template <class T, bool kDirect = false, class V, class F>
 __device__ __forceinline__ void product(const CgOperands& o, const LoopView& L, V v, F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (kDirect) {
+        ChunkCursor<T> cur(o, L);
+        walk_steps<T>(cur, v, [&](int k, T sum) {
+            const int row = (L.c0 + k) * kSellRows + lane;
+            if (row >= L.lo && row < L.hi) f(k * kSellRows + lane, row, sum);
+        });
+        return;
+    }
     const T* part = reinterpret_cast<const T*>(L.part);
     for (int k0 = 0; k0 < L.nc; k0 += L.tile) {
         const int k1 = min(L.nc, k0 + L.tile);
@@ -284,9 +354,21 @@ __device__ __forceinline__ void product(const CgOperands& o, const LoopView& L, 
 }
 
 // g(local row, row) for every row of the block, by the thread product() gives it to
-template <class G>
+template <bool kDirect = false, class G>
 __device__ __forceinline__ void own_rows(const CgOperands& o, const LoopView& L, G g) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (kDirect) {
+        for (int k0 = warp; k0 < L.nc; k0 += 32 * L.warps) {
+            const int q = k0 + lane * L.warps;
+            unsigned in = __ballot_sync(0xffffffffu, q < L.nc && o.loop_w[L.c0 + q] > 0);
+            for (; in != 0u; in &= in - 1u) {
+                const int k = k0 + (__ffs(static_cast<int>(in)) - 1) * L.warps;
+                const int row = (L.c0 + k) * kSellRows + lane;
+                if (row >= L.lo && row < L.hi) g(k * kSellRows + lane, row);
+            }
+        }
+        return;
+    }
     for (int k = warp; k < L.nc; k += L.warps) {
         const int row = chunk_of(L, k) * kSellRows + lane;
         if (row >= L.lo && row < L.hi) g(k * kSellRows + lane, row);

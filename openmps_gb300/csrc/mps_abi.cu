@@ -676,7 +676,8 @@ void read_status(mps_handle* h, bool solve_done) {
         if (h->direct_launches >= 0) {
             launched(h, static_cast<int>(h->direct_launches));
         } else if (h->cg.one_launch()) {
-            launched(h, one_launch_count(h->prm.solver, &h->mg, h->prm.solver != MPS_SOLVER_CG64));
+            launched(h, one_launch_count(h->prm.solver, &h->mg, h->prm.solver != MPS_SOLVER_CG64,
+                                         static_cast<int>(sell_chunks(h->n))));
         } else {
             const int kpi = h->cg.kernels_per_iteration(), kpu = h->cg.kernels_per_update();
             const int own = S.iter - S.fb_iter;
@@ -2005,7 +2006,7 @@ int mps_cg_solve_csr(mps_handle* h, int64_t n, const int64_t* row_ptr, const int
         check(cudaStreamSynchronize(s), "cg solve");
         if (iterations) *iterations = S.iter;
         if (true_relres) *true_relres = (S.bb > 0) ? std::sqrt(S.true_rr / S.bb) : std::sqrt(S.true_rr);
-        h->stats.kernel_launches += 1 + one_launch_count(solver, nullptr, false);
+        h->stats.kernel_launches += 1 + one_launch_count(solver, nullptr, false, o.nchunks);
         if (S.timed_out) throw StatusError{MPS_ERR_TIMEOUT, "a bounded wait of the solve timed out"};
         if (!S.converged)
             throw StatusError{MPS_ERR_CG_NOT_CONVERGED,

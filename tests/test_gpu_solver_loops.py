@@ -100,6 +100,31 @@ def test_loop_sizes(gpu_lib, name, solver):
     assert it2 == it and np.array_equal(x, again)  # every sum has a fixed order
 
 
+# past the rows whose chunks a block's tables surely hold: more chunks in the loop than the
+# tables (whole chunks walked, some left out, rows of one step and of several), and so many
+# left out that the tables hold the rest
+PAST_TABLES = {
+    "walked": dict(n=1_300_003, offsets=(1, 2, 3, 4, 5, 6)),
+    "walked_past_left_out": dict(n=3_200_001, offsets=(1,), identity=0.98),
+    "tables_hold_the_rest": dict(n=1_700_001, offsets=(1,), identity=0.98),
+}
+
+
+@pytest.mark.parametrize("solver", ["cg64", "mixed"])
+@pytest.mark.parametrize("name", list(PAST_TABLES))
+def test_past_the_tables(gpu_lib, name, solver):
+    from openmps_gb300.computer import Computer
+
+    ptr, col, val, b, xs, x0 = _system(seed=len(name), **PAST_TABLES[name])
+    c = Computer(abi.make_params())
+    which = abi.SOLVER_CG64 if solver == "cg64" else abi.SOLVER_MIXED
+    x, it, rel = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    assert rel <= 1.01e-12
+    assert float(np.linalg.norm(x - xs) / np.linalg.norm(xs)) <= TOL
+    again, it2, _ = c.cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS, solver=which)
+    assert it2 == it and np.array_equal(x, again)
+
+
 # every way the allocation-free solve walks its rows, around the largest system one cluster
 # takes (2,048 rows) and at the largest it accepts
 NOALLOC = {
