@@ -364,11 +364,18 @@ int g_loop_cluster = 0;    // blocks of the cluster form (0: a cluster of that s
 size_t g_loop_smem = 0;    // largest dynamic shared memory of a block
 
 // Chunks up to which the cluster form is used: its exchange is the cheaper one, but sixteen
-// SMs have a tenth of the FP64 pipes and of the loads in flight.  us per iteration, cluster
-// against grid (dam breaks at r_e = 4 l0; the WHILE node's kernels took 29-31 and 19-21):
-//   rows      1,850        3,133        5,250         9,403
-//   CG64    6.2 / 8.2    8.7 / 7.9   11.2 / 8.0    16.8 / 8.5
-//   MIXED   5.4 / 7.1    5.8 / 7.3    8.2 / 7.2    11.1 / 7.2
+// SMs have a tenth of the FP64 pipes and of the loads in flight.  And a cluster leaves the
+// chip to other streams: grids of all SMs take turns, so four handles stepped from four
+// threads take four times one's solve.  us a step, cluster against grid, of one handle and of
+// each of four at once (dam breaks, r_e in l0; with kernels per phase four CG64 handles took
+// 1,450 at 4,116 rows and 2.1 l0):
+//   CG64   4,116 rows 2.1: 1,334 / 1,603, 363 / 1,433   3,745 rows 4.0: 2,260 / 2,205, 597 / 2,010
+//          5,250 rows 2.1: 1,602 / 1,840, 424 / 1,721   5,250 rows 4.0: 3,004 / 2,667, 798 / 2,556
+//   MIXED  5,250 rows 2.1: 1,786 / 2,100, 472 / 1,966   5,250 rows 4.0: 3,745 / 4,051, 1,029 / 3,970
+//          a tall tank 6,925 rows 4.0: 2,925 / 2,697, 817 / 2,634
+// Past the cluster four handles at once gain nothing over one after the other (CG64 at 10,920,
+// 19,538 and 63,996 rows 2,697, 3,902 and 8,663 us a step each; kernels per phase 2,531, 3,664
+// and 7,736, alone 9,275, 11,773 and 19,710); half grids would, but cost one handle 7 to 28 %.
 // The grid form at 16,850, 42,226, 90,050 and 340,050 rows: CG64 9.4, 12.4, 18.4, 52.0
 // (WHILE: 30.4, 31.5, 37.2, 73.7), MIXED 7.7, 9.4, 14.0 (20.6, 21.7, 25.1); the FP64 pipe
 // bounds the large CG64 systems (one multiply-add per entry: 6.4 us at 90,050 rows), the
@@ -378,7 +385,7 @@ size_t g_loop_smem = 0;    // largest dynamic shared memory of a block
 // tile by tile in each product, and walked: 1.69 M rows of 28.9 entries 183 / 116, 170 / 134,
 // 139 / 92; 2.4 M of 13 203 / 125, 176 / 133, 128 / 77; 4 M of 13 273 / 186, 339 / 278,
 // 240 / 107 (DRAM's 6.8 TB/s bound these: 4 M rows are 624 / 416 MB of matrix an iteration).
-constexpr int kClusterChunks64 = 80, kClusterChunks32 = 128;
+constexpr int kClusterChunks64 = 128, kClusterChunks32 = 168;
 
 LoopPlan loop_plan(int nchunks, bool cluster, int keep_row_bytes) {
     LoopPlan p{};

@@ -545,9 +545,17 @@ size_t g_pcg_smem = 0;   // largest dynamic shared memory of a block
 // Rows of a full level-1 cell, about (21 in the dam breaks at rest).
 constexpr int kCellRows = 24;
 
-// Rows up to which the cluster form is used: us per solve, cluster against grid, 1,850 rows
-// 760 / 818, 3,133 rows 998 / 938, 5,250 rows 1,082 / 1,018, 9,403 rows 1,344 / 1,172.
-constexpr int kPcgClusterRows = 2560;
+// Rows up to which the cluster form is used, and those up to which the grid is half the SMs.
+// A grid of all SMs has the chip to itself: several handles' solves then take turns, where the
+// kernel chain overlapped them.  us a step of one handle and of each of four stepped from four
+// threads (dam breaks at r_e = 4 l0, another at 2.1, a tall tank):
+//   rows                4,116 (2.1)  5,250      6,925 (tall)  10,920      19,538 (2.1)  63,996 (2.1)
+//   cluster             895 / 249    1,068 / 304   1,186 / 345   1,465 / 423   1,870 / 525    -
+//   half the SMs        973 / 438    1,076 / 467   1,118 / 516   1,308 / 650   1,500 / 731   2,417 / 1,270
+//   all SMs             983 / 836    1,081 / 853   1,112 / 918   1,280 / 1,101 1,477 / 1,316 2,071 / 1,900
+//   chain (2.1)       1,789 / 511        -             -         2,167 / 625   2,345 / 759   2,680 / 1,068
+// Half the SMs cost one handle 1 to 3 % up to 20,000 rows and 17 % at 63,996.
+constexpr int kPcgClusterRows = 5376, kPcgHalfRows = 12288;
 
 // Largest level that every block takes by itself: a level costs 2,300 cycles per 512 cells
 // in one block, and two exchanges and its round trips (9,000 cycles) when it is distributed.
@@ -556,11 +564,10 @@ constexpr int kPcgClusterRows = 2560;
 // 1,172.
 constexpr int kPcgBottomCells = 2048;
 
-bool pcg_plan(const MgHierarchy& mg, bool cluster, PcgPlan* plan) {
-    if (mg.levels <= 0 || mg.n <= 0) return false;
+bool pcg_plan(const MgHierarchy& mg, int blocks, PcgPlan* plan) {
+    if (mg.levels <= 0 || mg.n <= 0 || blocks <= 0) return false;
     PcgPlan p{};
-    p.blocks = cluster ? kLoopCluster : g_pcg_sms;
-    if (p.blocks <= 0) return false;
+    p.blocks = blocks;
     const int each = mg.n / p.blocks + 1;
     p.rows = (each + each / 2 + 64 + 3) & ~3;
     p.tables = 2 * each / kSellRows + 4;
@@ -582,6 +589,12 @@ bool pcg_plan(const MgHierarchy& mg, bool cluster, PcgPlan* plan) {
     if (p.bottom > mg.levels) return false;
     *plan = p;
     return true;
+}
+
+// The form the rows take, where its blocks' shares fit.
+bool pcg_choose(const MgHierarchy& mg, PcgPlan* plan, bool* cluster) {
+    *cluster = g_pcg_cluster && mg.n <= kPcgClusterRows && pcg_plan(mg, kLoopCluster, plan);
+    return *cluster || (mg.n <= kPcgHalfRows && pcg_plan(mg, g_pcg_sms / 2, plan)) || pcg_plan(mg, g_pcg_sms, plan);
 }
 
 }  // namespace
@@ -626,13 +639,14 @@ cudaError_t pcg_loop_prepare_device() {
 
 bool pcg_loop_fits(const MgHierarchy& mg) {
     PcgPlan p;
-    return mg.cell_w != nullptr && pcg_plan(mg, false, &p);
+    bool cluster;
+    return mg.cell_w != nullptr && pcg_choose(mg, &p, &cluster);
 }
 
 cudaError_t launch_pcg_loop(const CgOperands& o, const MgHierarchy& mg, cudaStream_t s) {
     PcgPlan p;
-    const bool cluster = g_pcg_cluster && mg.n <= kPcgClusterRows && pcg_plan(mg, true, &p);
-    if (!cluster && !pcg_plan(mg, false, &p)) return cudaErrorInvalidValue;
+    bool cluster;
+    if (!pcg_choose(mg, &p, &cluster)) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(p.blocks));
     cfg.blockDim = dim3(kLoopThreads);

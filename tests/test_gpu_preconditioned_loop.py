@@ -56,3 +56,57 @@ def test_loop_matches_cg(gpu_lib, name):
     again, st2 = _step(s, solver=abi.SOLVER_MIXED_MG, re_by_l0=radius)
     assert st2["cg_iterations"] == st["cg_iterations"]
     np.testing.assert_array_equal(mg, again)  # every sum has a fixed order
+
+
+# around the largest scenes of one cluster (5,376 rows) and of half the SMs (12,288)
+FORMS = {
+    "cluster_5250": (5e-3, 0.2, 0.4, 0.8, 0.6, 4.0),
+    "half_5961": (4.6e-3, 0.2, 0.4, 0.8, 0.6, 4.0),
+    "half_10875": (3e-3, 0.06, 1.0, 0.1, 1.2, 4.0),
+    "grid": (2.9e-3, 0.2, 0.4, 0.8, 0.6, 4.0),
+}
+
+
+@pytest.mark.parametrize("name", list(FORMS))
+def test_forms_match_cg(gpu_lib, name):
+    l0, ww, wh, tw, th, radius = FORMS[name]
+    s = scenes.dam_break(l0, ww, wh, tw, th)
+    mg, st = _step(s, solver=abi.SOLVER_MIXED_MG, re_by_l0=radius)
+    cg, _ = _step(s, solver=abi.SOLVER_CG64, re_by_l0=radius)
+    n = wh / l0
+    print("%s: %d particles" % (name, s.count))
+    assert st["fallback"] == 0 and st["cg_true_relres"] <= 1e-10
+    assert float(np.linalg.norm(mg - cg) / np.linalg.norm(cg)) <= 2e-10 * 7 * n * n
+    again, _ = _step(s, solver=abi.SOLVER_MIXED_MG, re_by_l0=radius)
+    np.testing.assert_array_equal(mg, again)
+
+
+def test_handles_at_once(gpu_lib):
+    # four handles stepped from four threads end where one by itself does, in each form
+    import threading
+
+    from openmps_gb300.computer import Computer
+
+    for l0 in (5e-3, 3.6e-3, 2.5e-3):
+        s = scenes.dam_break(l0, 0.2, 0.4, 0.8, 0.6)
+        cs = []
+        for _ in range(5):
+            c = Computer(s.params(criterion=abi.CRIT_RHS, eps=1e-10, solver=abi.SOLVER_MIXED_MG))
+            c.add_scene(s)
+            cs.append(c)
+
+        def go(c):
+            for _ in range(4):
+                c.forward_time(0.01 * l0)
+
+        go(cs[0])
+        threads = [threading.Thread(target=go, args=(c,)) for c in cs[1:]]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        want = cs[0].particles()
+        for c in cs[1:]:
+            got = c.particles()
+            for k in ("x", "z", "u", "w", "p"):
+                np.testing.assert_array_equal(got[k], want[k], err_msg=k)

@@ -125,6 +125,17 @@ def test_past_the_tables(gpu_lib, name, solver):
     assert it2 == it and np.array_equal(x, again)
 
 
+@pytest.mark.parametrize("n", [168 * 32, 168 * 32 + 1])
+def test_mixed_cluster_edge(gpu_lib, n):
+    from openmps_gb300.computer import Computer
+
+    ptr, col, val, b, xs, x0 = _system(n, (1, 2, 73, 74), seed=n)
+    x, _, rel = Computer(abi.make_params()).cg_solve_csr(ptr, col, val, b, x0, 1e-12, criterion=abi.CRIT_RHS,
+                                                         solver=abi.SOLVER_MIXED)
+    assert rel <= 1.01e-12
+    assert np.linalg.norm(x - xs) <= TOL * np.linalg.norm(xs)
+
+
 # every way the allocation-free solve walks its rows, around the largest system one cluster
 # takes (2,048 rows) and at the largest it accepts
 NOALLOC = {
