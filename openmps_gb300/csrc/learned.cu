@@ -16,6 +16,7 @@
 // network output.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -474,6 +475,7 @@ constexpr int kTrainThreads = 256;
 constexpr int kTrainS = 32;         // samples of a block
 constexpr int kTileS = 64;          // samples of a cluster of two
 constexpr int kTrainClusters = 76;  // a block per SM
+constexpr int kTrainParts = 148;    // partial gradients of a large batch
 // floats of a 64-unit and a 16-feature row in shared memory: 16-byte aligned, rows shifted by
 // four banks
 constexpr int kPitch = 68, kPitchX = 20;
@@ -608,15 +610,17 @@ __device__ __forceinline__ void dense_wgrad(const float* Delta, const float* In,
 }
 
 // Losses of `n` samples (rows order[0 .. n - 1] of `samples`, or its first n rows without an
-// order) and the gradient of their mean; one partial gradient per cluster.
+// order) and the gradient of their mean: `parts` partial gradients, part p of the tiles p,
+// p + parts, .. in FP32 (kTrainParts parts whatever the grid: fewer make longer FP32 sums).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads)
     k_mlp_grad(const float* __restrict__ w, const float* __restrict__ samples, const int64_t* __restrict__ order,
-               int64_t n, float* partials, float* losses) {
+               int64_t n, int parts, float* partials, float* losses) {
     extern __shared__ __align__(16) float sh[];
     const int t = threadIdx.x, rank = static_cast<int>(blockIdx.x & 1u), row0 = kTrainS * rank;
     PairMem M{sh, smem_u32(sh)};
     asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(M.peer) : "r"(rank ^ 1));
-    const int64_t stride = static_cast<int64_t>(gridDim.x >> 1) * kTileS;
+    const int clusters = static_cast<int>(gridDim.x >> 1);
+    const int64_t stride = static_cast<int64_t>(parts) * kTileS;
     const int fk = t & 15;  // the feature this thread loads
     // features of this block's samples (t >> 4) and (t >> 4) + 16, y or g of threads fk < 2
     float feat[2], target[2];
@@ -633,7 +637,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads)
             target[q] = row[q] >= 0 && fk < 2 ? samples[row[q] * kMlpSampleFloats + 16 + fk] : 0.0f;
         }
     };
-    int64_t tile = static_cast<int64_t>(blockIdx.x >> 1) * kTileS;
+    int part = static_cast<int>(blockIdx.x >> 1);
+    int64_t tile = static_cast<int64_t>(part) * kTileS;
     fetch(tile);
     pdl_begin();  // the weights come from the update just before
     {
@@ -675,7 +680,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads)
     float g2[2][4] = {}, g3[2][4] = {}, g1[2] = {};
     float gb = 0.0f, g4 = 0.0f, gb4 = 0.0f;
     const float inv_total = 1.0f / static_cast<float>(n);
-    for (; tile < n; tile += stride) {
+    while (tile < n) {
+        int64_t next = tile + stride;  // the part's next tile, or the first of the cluster's next part
+        const bool last = next >= n;
+        if (last) next = part + clusters < parts ? static_cast<int64_t>(part + clusters) * kTileS : n;
         pair_barrier();  // the peer has started, and is done with the tile before
 #pragma unroll
         for (int q = 0; q < 2; q++) {
@@ -685,7 +693,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads)
         }
         __syncthreads();
         dense_fwd<16, kPitchX>(M, row0, kTrX, kTrWt1, kTrB, kTrA1, kTrD1);
-        if (tile + stride < n) fetch(tile + stride);
+        if (next < n) fetch(next);
         __syncthreads();
         dense_fwd<64, kPitch>(M, row0, kTrA1, kTrWt2, kTrB + 64, kTrA2, kTrD2);
         __syncthreads();
@@ -765,21 +773,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads)
             for (int s = 0; s < kTileS; s++) b += sh[kTrO + 2 * s + rank];
             gb4 += b;
         }
-    }
-    float* dst = partials + static_cast<int64_t>(blockIdx.x >> 1) * kMlpParams;
+        if (last) {
+            float* dst = partials + static_cast<int64_t>(part) * kMlpParams;
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
+            for (int i = 0; i < 2; i++) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            dst[gW2 + (gj + i) * 64 + gk + k] = g2[i][k];
-            dst[gW3 + (gj + i) * 64 + gk + k] = g3[i][k];
+                for (int k = 0; k < 4; k++) {
+                    dst[gW2 + (gj + i) * 64 + gk + k] = g2[i][k];
+                    dst[gW3 + (gj + i) * 64 + gk + k] = g3[i][k];
+                }
+            }
+            dst[gW1 + 16 * row0 + 2 * t] = g1[0];
+            dst[gW1 + 16 * row0 + 2 * t + 1] = g1[1];
+            if (t < 96) dst[(t < 32 ? gB1 : t < 64 ? gB2 : gB3) + row0 + (t & 31)] = gb;
+            else if (t >= 128 && t < 192) dst[gW4 + 64 * rank + t - 128] = g4;
+            else if (t == 192) dst[gB4 + rank] = gb4;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) g2[i][k] = g3[i][k] = 0.0f;
+                g1[i] = 0.0f;
+            }
+            gb = g4 = gb4 = 0.0f;
+            part += clusters;
         }
+        tile = next;
     }
-    dst[gW1 + 16 * row0 + 2 * t] = g1[0];
-    dst[gW1 + 16 * row0 + 2 * t + 1] = g1[1];
-    if (t < 96) dst[(t < 32 ? gB1 : t < 64 ? gB2 : gB3) + row0 + (t & 31)] = gb;
-    else if (t >= 128 && t < 192) dst[gW4 + 64 * rank + t - 128] = g4;
-    else if (t == 192) dst[gB4 + rank] = gb4;
 }
 
 // The draws of one Fisher-Yates shuffle of 0 .. n - 1 by SplitMix64 (Steele, Lea, Flood
@@ -842,7 +861,7 @@ __global__ void __launch_bounds__(kUpdateThreads) k_mlp_update(const float* part
     }
     const int e = blockIdx.x * 32 + lane;
     // all of the warp's partials in flight, then two chains of additions
-    constexpr int kMost = (kTrainClusters + 7) / 8;
+    constexpr int kMost = (kTrainParts + 7) / 8;
     float x[kMost];
 #pragma unroll
     for (int k = 0; k < kMost; k++) {
@@ -949,12 +968,13 @@ void launch_mlp_infer(const void* packed, const float* feat, int n, const double
 
 int mlp_train_partials(int64_t n) {
     const int64_t c = (n + kTileS - 1) / kTileS;
-    return static_cast<int>(c < kTrainClusters ? (c > 0 ? c : 1) : kTrainClusters);
+    return static_cast<int>(c < kTrainParts ? (c > 0 ? c : 1) : kTrainParts);
 }
 
 void launch_mlp_loss_grad(const MlpTrainer& T, const float* samples, int64_t n, cudaStream_t s) {
     const int parts = mlp_train_partials(n);
-    k_mlp_grad<<<2 * parts, kTrainThreads, kTrBytes, s>>>(T.w, samples, nullptr, n, T.partials, T.losses);
+    k_mlp_grad<<<2 * std::min(parts, kTrainClusters), kTrainThreads, kTrBytes, s>>>(T.w, samples, nullptr, n, parts,
+                                                                                T.partials, T.losses);
     k_mlp_update<false><<<kUpdateBlocks + 1, kUpdateThreads, 0, s>>>(T.partials, parts, T.losses, n, T.grad, T.loss,
                                                                    nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f);
 }
@@ -968,7 +988,8 @@ void launch_mlp_train_step(const MlpTrainer& T, const int64_t* order, int64_t n,
     const float bc1 = 1.0f - std::pow(0.9f, static_cast<float>(step));
     const float bc2 = 1.0f - std::pow(0.999f, static_cast<float>(step));
     const int parts = mlp_train_partials(n);
-    launch_pdl(k_mlp_grad, 2 * parts, kTrainThreads, kTrBytes, s, T.w, T.samples, order, n, T.partials, T.losses);
+    launch_pdl(k_mlp_grad, 2 * std::min(parts, kTrainClusters), kTrainThreads, kTrBytes, s, T.w, T.samples, order, n,
+               parts, T.partials, T.losses);
     launch_pdl(k_mlp_update<true>, kUpdateBlocks + 1, kUpdateThreads, 0, s, T.partials, parts, T.losses, n, nullptr,
                loss, T.w, T.m, T.v, lr, bc1, bc2);
 }

@@ -40,6 +40,27 @@ def test_gradient_matches_oracle(gpu_lib, n):
     assert err < 1e-4, err
 
 
+@pytest.mark.parametrize("n", [4096, 8192, 16384, 32768])
+def test_gradient_of_large_batches_sums_148_parts(gpu_lib, n):
+    # A batch's gradient is its tiles' (64 samples) in at most 148 FP32 sums of tiles 148
+    # apart, then FP64 over those (each eighth one in one of eight sums, even and odd ones
+    # apart): composed here from the gradients of the tiles by themselves.  n / 64 is a power
+    # of two, so 1 / 64 against 1 / n scales every term exactly, and the bits are the same.
+    blob, samples = _random_case(3, n)
+    _, got = mlp_loss_grad(blob, samples)
+    tiles = [mlp_loss_grad(blob, samples[k:k + 64])[1] for k in range(0, n, 64)]
+    parts = []
+    for p in range(min(148, len(tiles))):
+        g = np.zeros_like(got)
+        for k in range(p, len(tiles), 148):
+            g = g + tiles[k]
+        parts.append(g.astype(np.float64))
+    zero = np.zeros(got.size)
+    warps = [sum(parts[w::16], zero) + sum(parts[w + 8::16], zero) for w in range(8)]
+    total = ((warps[0] + warps[1]) + (warps[2] + warps[3])) + ((warps[4] + warps[5]) + (warps[6] + warps[7]))
+    np.testing.assert_array_equal(got, (total * (64.0 / n)).astype(np.float32))
+
+
 @pytest.mark.parametrize("n,batch", [(1, 4), (31, 31), (33, 64), (64, 64), (130, 64), (5000, 4900)])
 def test_training_steps_match_oracle(gpu_lib, n, batch):
     # Three epochs of the same minibatches in FP64 (the shuffle by SplitMix64 and Fisher-Yates).
