@@ -55,8 +55,8 @@ __global__ void k_bucket(SceneConst sc, DeviceState st) {
 __global__ void __launch_bounds__(kBlock) k_cell_sort(SceneConst sc, DeviceState st) {
     constexpr int kMost = 64;
     __shared__ int buf[kBlock / kLanes][kMost];
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = t / kLanes, g = t & (kLanes - 1);
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // 8 per cell: past 2^31
+    const int c = static_cast<int>(t / kLanes), g = threadIdx.x & (kLanes - 1);
     int* b = buf[threadIdx.x / kLanes];
     int cnt = 0;
     int32_t* s = st.cell_slot;
