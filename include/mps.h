@@ -90,10 +90,13 @@ extern "C" {
  * reference, whose CG is unpreconditioned. */
 #define MPS_SOLVER_MIXED_MG 3
 
-/* How the CG loop is launched: one CUDA graph with a device-driven while loop, or
- * host-launched kernel batches (the same kernels; for profilers that cannot see
- * kernels inside conditional graphs). */
-#define MPS_CG_LAUNCH_GRAPH 0   /* one CUDA graph per solve, every phase its own kernel */
+/* How the CG loop is launched: one CUDA graph (the iterations in one launch, or, for
+ * preconditioned systems past about 120,000 rows, kernels per phase under a device-driven
+ * while loop), or the same kernels launched by the host (for profilers that cannot see
+ * kernels inside conditional graphs).  A loop in one launch is a cluster of 16 blocks for
+ * small systems, else a cooperative grid that starts when all its SMs have room: solves of
+ * several handles at once then take turns. */
+#define MPS_CG_LAUNCH_GRAPH 0   /* one CUDA graph per solve */
 #define MPS_CG_LAUNCH_HOST 1
 #define MPS_CG_LAUNCH_GRAPH_KERNELS 0  /* the same as MPS_CG_LAUNCH_GRAPH */
 #define MPS_CG_LAUNCH_PERSISTENT 2     /* MIXED_MG / LEARNED: the iterations in one persistent
@@ -271,8 +274,10 @@ int mps_event_elapsed(mps_handle* h, int32_t begin, int32_t end, float* ms);
 /* Writes `bytes` of scratch on the handle's stream, then reads it back: evicts L2 between
  * timed runs and leaves it holding clean lines, so the timed work writes nothing back. */
 int mps_flush_l2(mps_handle* h, int64_t bytes);
-/* Times the PPE solver's SpMV kernel alone on the last assembled matrix: `reps`
- * back-to-back launches (FP64 values for MPS_SOLVER_CG64, FP32 for MPS_SOLVER_MIXED);
+/* Times one product with the last assembled matrix as a kernel by itself: `reps`
+ * back-to-back launches (FP64 values for MPS_SOLVER_CG64, FP32 for MPS_SOLVER_MIXED; the
+ * preconditioned kernel chain's own SpMV for MPS_SOLVER_MIXED_MG.  The single-launch loops
+ * form their products inside);
  * *ms_per_launch receives the mean CUDA-event time of one launch.  When flush_bytes
  * > 0, L2 is flushed before every launch and only the launch is timed. */
 int mps_bench_spmv(mps_handle* h, int32_t solver, int32_t reps, int64_t flush_bytes,

@@ -146,10 +146,6 @@ __device__ bool grid_sum(double a, double b, double c, double* partials, uint32_
     return true;
 }
 
-__device__ __forceinline__ bool cg_done(const CgScalars* S) {
-    return S->converged || S->aborted || S->iter >= S->max_iter;
-}
-
 // One warp per chunk of kSellRows rows (lane = row within the chunk).  The SpMV kernels
 // launch as many warps as chunks so the block scheduler balances uneven chunks.
 struct ChunkLoop {
@@ -226,7 +222,7 @@ __device__ __forceinline__ void pad_row(const CgOperands& o, int c, int i, int L
 }
 
 // ------------------------------------------------------------- CG64 kernels
-// Ap = A x; r = b - Ap; p = r; rr = r.r (Computer.hpp:1382-1385).  With `gate` (the
+// r = b - A x; rr = r.r (Computer.hpp:1382-1385; the loop starts from p = 0, beta = 0).  With `gate` (the
 // fallback after a preconditioned solve) nothing runs unless that solve failed.
 __global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, const CgScalars* gate) {
     __shared__ BlockTicket tk;
@@ -255,7 +251,6 @@ __global__ void __launch_bounds__(kBlock) k_cg_init(CgOperands o, const CgScalar
             const double bi = o.b[i];
             ri = bi - ax;
             o.r[i] = ri;
-            o.p[i] = ri;
             vrr += ri * ri;
             vbb += bi * bi;
         }
@@ -632,24 +627,20 @@ struct StageRing {
     }
 };
 
-// What a staged FP64 SpMV computes: the CG's A p (with p.Ap and the step size alpha =
-// rr / p.Ap), or the mixed solves' true residual r = b - A x' after a
-// reliable update folded the FP32 correction into x' (with r.r and the update's decisions).
-enum StagedKind { kStagedCgAp = 0, kStagedTrueResidual = 1 };
+// What a staged FP64 SpMV computes: the preconditioned solves' true residual r = b - A x'
+// after a reliable update folded the FP32 correction into x' (with r.r and the update's
+// decisions), or A r and r.A r by itself, which mps_bench_spmv times (the plain solvers form
+// that product inside their loops, cgloop.cuh).
+enum StagedKind { kStagedProduct = 0, kStagedTrueResidual = 1 };
 
-// A lane sums its row from the stages in
-// ascending column order with one accumulator (the order of row64), so the row sums are
-// those of the per-chunk kernel.
+// A lane sums its row from the stages in ascending column order with one accumulator (the
+// order of row64), so the row sums are those of the per-chunk kernels.
 template <int SLICE, int STAGES, int MINB, int KIND>
 __global__ void __launch_bounds__(kStgThreads, MINB) k_cg_spmv_dot_staged(CgOperands o, cudaGraphConditionalHandle h,
                                                                           int use_cond) {
     extern __shared__ __align__(128) unsigned char stg_sm[];
     __shared__ BlockTicket tk;
-    if (KIND == kStagedCgAp) {
-        if (cg_done(o.S)) return;
-    } else if (o.S->converged || o.S->aborted || o.S->stalled || !o.S->do_update) {
-        return;
-    }
+    if (KIND == kStagedTrueResidual && (o.S->converged || o.S->aborted || o.S->stalled || !o.S->do_update)) return;
     ticket_init(tk);
     using Ring = StageRing<SLICE, STAGES, 2>;
     constexpr int kStageBytes = Ring::kEntries * 12;
@@ -664,8 +655,8 @@ __global__ void __launch_bounds__(kStgThreads, MINB) k_cg_spmv_dot_staged(CgOper
            reinterpret_cast<uint64_t*>(stg_sm + static_cast<size_t>(kStgWarps) * STAGES * kStageBytes) + w * STAGES,
            gw);
     for (int k = 0; k < STAGES; k++) R.issue(o, nw);
-    // the gathered vector: p, or the folded solution x' (the buffer the update writes)
-    const double* __restrict__ p = KIND == kStagedCgAp ? o.p : ((o.S->updates & 1) != 0 ? o.x : o.x2);
+    // the gathered vector: r, or the folded solution x' (the buffer the update writes)
+    const double* __restrict__ p = KIND == kStagedProduct ? o.r : ((o.S->updates & 1) != 0 ? o.x : o.x2);
     double v = 0.0;
     int item = 0;
     bool ok = true;
@@ -709,7 +700,7 @@ __global__ void __launch_bounds__(kStgThreads, MINB) k_cg_spmv_dot_staged(CgOper
         }
         if (!ok) break;
         if (i < o.n) {
-            if (KIND == kStagedCgAp) {
+            if (KIND == kStagedProduct) {
                 o.Ap[i] = acc;
                 v += p[i] * acc;
             } else {
@@ -723,12 +714,10 @@ __global__ void __launch_bounds__(kStgThreads, MINB) k_cg_spmv_dot_staged(CgOper
     if (grid_sum(v, 0.0, 0.0, o.partials, o.tickets, &o.S->counter, tk, tot)) {
         CgScalars* S = o.S;
         S->counter = 0;
-        if (KIND == kStagedCgAp) {
+        if (KIND == kStagedProduct)
             S->pAp = tot[0];
-            S->alpha = S->rr / tot[0];
-        } else {
+        else
             true_residual_done(S, tot[0], h, use_cond);
-        }
         if (o.status && (o.status->flags & kStatusWaitTimeout)) S->aborted = 1;
     }
 }
@@ -761,9 +750,9 @@ int staged_grid(const CgOperands& o) {
     return need < cap ? (need > 0 ? need : 1) : cap;
 }
 
-// the FP64 CG's SpMV (Ap = A p, p.Ap, alpha)
-void launch_cg_spmv(const CgOperands& o, cudaStream_t s) {
-    k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedCgAp>
+// the FP64 product by itself (Ap = A r, r.Ap)
+void launch_spmv64(const CgOperands& o, cudaStream_t s) {
+    k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedProduct>
         <<<staged_grid(o), kStgThreads, kStgSmem64, s>>>(o, 0, 0);
 }
 
@@ -1210,7 +1199,7 @@ int cg_grid_vec(int64_t n) { return grid_for(n); }
 int cg_grid_spmv(int64_t n) { return grid_for(sell_chunks(n) * 32); }
 
 cudaError_t cg_prepare_device() {
-    auto k = k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedCgAp>;
+    auto k = k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedProduct>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kStgSmem64));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_cg_spmv_dot_staged<kStgSlice64, kStgStages64, kStgBlocks64, kStagedTrueResidual>,
@@ -1241,7 +1230,7 @@ void launch_cg_configure(CgScalars* S, double eps, int criterion, int max_iter, 
 
 void launch_spmv_only(int solver, const CgOperands& ops, cudaStream_t s) {
     if (solver == MPS_SOLVER_CG64)
-        launch_cg_spmv(ops, s);
+        launch_spmv64(ops, s);
     else if (is_pcg(solver))
         launch_pmx_spmv(ops, 1, 0, 0, 0, s, false);
     else
@@ -1294,7 +1283,8 @@ cudaError_t fallback_kernels(const CgOperands& ops, const CgOperands& fb, int af
 
 namespace {
 // Whether the solver's iteration loop is one launch: where its block's share fits shared
-// memory it was faster at every size measured (pcgloop.cu).
+// memory it was faster than kernels per phase at every size measured (1,850 to 127,260 rows,
+// whose step took 3,001 us against 3,563; CG64 and MIXED to 4 M rows, cgloop.cu).
 bool loops_in_one_launch(int solver, const MgHierarchy* mg) {
     return !is_pcg(solver) || pcg_loop_fits(*mg);
 }

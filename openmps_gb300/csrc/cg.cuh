@@ -243,9 +243,9 @@ struct LearnedRun {
     CgScalars* S;
 };
 
-// A CUDA graph running one whole solve: init kernels + the iteration loop (one launch for
-// the plain solvers, a device-driven while loop for the preconditioned ones) + for the
-// mixed-precision solvers the FP64 CG fallback loop, which runs only after a failure.
+// A CUDA graph running one whole solve: init kernels + the iteration loop (one launch; for
+// preconditioned systems whose blocks' shares do not fit that, a device-driven while loop) +
+// for the mixed-precision solvers the FP64 CG fallback loop, which runs only after a failure.
 // Side stream and events of a fork/join inside a captured graph.
 struct SetupFork {
     cudaStream_t side = nullptr;
@@ -306,7 +306,7 @@ int one_launch_count(int solver, const MgHierarchy* mg, bool with_fb, int nchunk
 // Sets eps / criterion / max_iter / delta for the next solve (stream-ordered).
 void launch_cg_configure(CgScalars* S, double eps, int criterion, int max_iter, double delta2,
                          cudaStream_t s);
-// One launch of the solver's SpMV kernel (the CG iteration's dominant kernel) alone.
+// One product with the matrix as a kernel by itself (mps_bench_spmv).
 void launch_spmv_only(int solver, const CgOperands& ops, cudaStream_t s);
 // Shared-memory opt-in of the staged SpMV kernels (once per device, before they launch).
 cudaError_t cg_prepare_device();

@@ -814,15 +814,6 @@ __global__ void __launch_bounds__(256) k_mlp_draws(uint64_t state, int64_t n, in
     pick[i] = static_cast<int64_t>(z % static_cast<uint64_t>(i + 1));
 }
 
-// A float as a double (exact) on the integer pipe: a conversion takes GB300's FP64 pipe as
-// long as an addition.  Zeros, subnormals, infinities and NaN are converted there.
-__device__ __forceinline__ double widen(float f) {
-    const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu;
-    if (e == 0u || e == 255u) return static_cast<double>(f);
-    return __hiloint2double(static_cast<int>((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)),
-                            static_cast<int>(u << 29));
-}
-
 // grad = sum of the block partials in a fixed order (FP64), loss likewise; with kAdam the
 // Adam step of the entry follows.  32 entries a block, eight warps sharing the partials:
 // one thread per entry took 13.4 us for 64 partials (a chain of FP64 additions) and Adam
