@@ -506,8 +506,10 @@ void allocate(mps_handle* h, int64_t n, int64_t keep) {
     h->psync.gen = dalloc<unsigned>(h, 1);
     h->psync.err = dalloc<int32_t>(h, 1);
     h->psync.limits = h->d_limits;
-    h->psync.blocks = persistent_blocks();
-    h->psync.partials = dalloc<double>(h, 3 * static_cast<int64_t>(h->psync.blocks));
+    if (h->prm.cg_launch == MPS_CG_LAUNCH_PERSISTENT) {  // set for the handle's life
+        h->psync.blocks = persistent_blocks();
+        h->psync.partials = dalloc<double>(h, 3 * static_cast<int64_t>(h->psync.blocks));
+    }
     cudaStream_t s = h->stream;
     // zero everything persistent, then carry the old contents over
     check(cudaMemsetAsync(st.type, 0, sizeof(int32_t) * n, s), "memset");
