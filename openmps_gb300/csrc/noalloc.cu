@@ -51,7 +51,8 @@ constexpr int64_t kNoallocDoubles = 3 * kNoallocMaxRows + kLoopSlots + kNoallocS
 // before and now: 500 rows of 13 entries 23.1 -> 5.5 and 2,000 of 48 30.9 -> 8.9 (cluster);
 // 3,600 of 13 22.4 -> 7.7, 10,000 of 28 25.7 -> 9.5, 100,441 of 5 / 28 / 48 21.5 -> 10.3,
 // 31.1 -> 17.9 and 44.1 -> 24.0 (grid: two exchanges of about 3 us, then the FP64 pipe, 5.3
-// us at 28 entries).
+// us at 28 entries).  Cluster / grid on either side of the line, 27 entries: 900 rows 6.3 / 7.3,
+// 2,025 7.3 / 7.4, 4,096 9.6 / 7.6, 8,100 13.0 / 9.3.
 constexpr int64_t kNoallocClusterRows = 2048;
 
 struct NoallocScalars {
