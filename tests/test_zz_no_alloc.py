@@ -144,6 +144,8 @@ class _GreenStream:
 
     def _ok(self, name, *args):
         rc = getattr(self.cu, name)(*args)
+        if rc == 801:  # CUDA_ERROR_NOT_SUPPORTED
+            pytest.skip("no green contexts here")
         assert rc == 0, (name, rc)
 
     def close(self):
